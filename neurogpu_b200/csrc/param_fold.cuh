@@ -26,6 +26,15 @@ NGPU_HD R pload(const float* __restrict__ pr, int q) {
     else return (R)pr[q * 32];
 }
 
+// x to the power of parameter P, loaded as q
+template <typename R, int P>
+NGPU_HD R ppow(R x, R q) {
+    if constexpr (ParamFold<P>::on) {
+        if constexpr (ParamFold<P>::v == 1.f) return x;
+    }
+    return Math<R>::pw(x, q);
+}
+
 // parameters B .. B+N-1 at rows q .. q+N-1 into out[0..N)
 template <typename R, int B, int N, int K = 0>
 NGPU_HD void pload_n(const float* __restrict__ pr, int q, R* out) {
