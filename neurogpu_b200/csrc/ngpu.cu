@@ -434,17 +434,16 @@ struct ngpu_sim {
     uint2* d_prange = nullptr;    // [ptab_rows] bit-pattern range of each parameter row
     unsigned long long* d_phash = nullptr;  // [ptab_rows] hash of each parameter row
     std::vector<int32_t> prow_canon;  // parameter block start -> the block it reads (identical values)
-    bool ch_prefetch = true;      // the runtime-specialised kernel compiles the channel-pass L2 prefetch in
     int layout = NGPU_LAYOUT_LANE_INSTANCE;  // lane = instance, or one warp per instance (thread-item)
     int ti_warps = 4;             // thread-item layout: instances (warps) per CTA
     int ti_items = 32;            // thread-item layout: work items per instance's tree
 };
 
-// Rows (state and parameter) a node's channel update reads, on average; the
-// channel-pass prefetch is compiled in from kPrefetchRowsPerNode on.  Measured
-// on B200: the HH-type cells (~30 rows per node) run 7-13 % faster with it,
-// the TTPC-like cell (~12) 7 % faster without it.
-constexpr double kPrefetchRowsPerNode = 20.0;
+// Rows (state and parameter) a node's channel update reads, on average, from
+// which on the tree is split into 2 items per warp instead of 3 (8-warp CTAs).
+// Measured on B200: the HH-type cells (~30 rows per node) run 9 % faster with
+// 2, the TTPC-like cell (~12) 5 % faster with 3.
+constexpr double kHeavyRowsPerNode = 20.0;
 
 // Thread-item layout: work items per instance at most / by default, and the
 // SM count the default CTA shape spreads a small batch over.
@@ -1070,11 +1069,7 @@ int ngpu_sim_create_layout(ngpu_model* m, int32_t n_sets, int32_t n_stim, int32_
     if (n_warps > 0) W = n_warps;
     W = std::min(W, m->n);
     s->n_warps = W;
-    s->ch_prefetch = rows_per_node(m) >= kPrefetchRowsPerNode;
-    if (const char* ev = getenv("NGPU_CH_PREFETCH")) s->ch_prefetch = atoi(ev) != 0;
-    // without the prefetch, finer items balance better (TTPC-like: +4 % from 2 to 3 per warp);
-    // the autotuner searches this per morphology
-    s->items_per_warp = s->ch_prefetch ? 2 : 3;
+    s->items_per_warp = rows_per_node(m) >= kHeavyRowsPerNode ? 2 : 3;
     if (const char* ev = getenv("NGPU_ITEMS_PER_WARP")) s->items_per_warp = std::max(1, std::min(8, atoi(ev)));
     if (items_per_warp > 0) s->items_per_warp = items_per_warp;
     if (ti) {
@@ -1386,14 +1381,11 @@ int ngpu_sim_set_recording(ngpu_sim* s, int32_t n_rec, const int32_t* rec_nodes,
 }
 
 // The mechanism masks a simulation's (or batch's) kernel is compiled for.
-// Whether the kernel is compiled without the generic channel path: only
-// when the compiled classes hold every mask in `all` (no node takes it), and
-// only for kernels without the channel-pass prefetch.  Measured on B200:
-// without the path the TTPC-like cell runs 6 % faster and the TTPC set
-// generated from its .mod files 16 % (its generic path alone made it spill);
-// the HH-type cells, compiled with the prefetch, run 2-4 % slower.
-static bool masks_cover(const std::vector<uint32_t>& picked, const std::vector<uint32_t>& all, bool prefetch) {
-    if (prefetch) return false;
+// Whether the kernel is compiled without the generic channel path: when the
+// compiled classes hold every mask in `all` (no node takes it).  Measured on
+// B200: without the path the TTPC-like cell runs 6 % faster and the TTPC set
+// generated from its .mod files 16 % (its generic path alone made it spill).
+static bool masks_cover(const std::vector<uint32_t>& picked, const std::vector<uint32_t>& all) {
     for (uint32_t x : all)
         if (std::find(picked.begin(), picked.end(), x) == picked.end()) return false;
     return true;
@@ -1517,7 +1509,7 @@ static int sim_upload_nodes(ngpu_sim* s) {
         } else {
             const std::vector<uint32_t> all = model_masks(m), picked = ngpu_jit::pick_masks(all, kMaxClasses);
             s->jit = ngpu_jit::module(m->mechset, s->precision == NGPU_FP64, picked, gs ? &gs->source : nullptr,
-                                      s->ch_prefetch, s->folds, masks_cover(picked, all, s->ch_prefetch),
+                                      s->folds, masks_cover(picked, all),
                                       s->layout == NGPU_LAYOUT_WARP_INSTANCE,
                                       s->layout == NGPU_LAYOUT_LANE_INSTANCE ? std::max(8, s->n_warps) : 8,
                                       wide_ctas_per_sm(s->n_groups));
@@ -1649,15 +1641,13 @@ static int batch_select_kernels(ngpu_batch* b) {
     b->jit = nullptr;
     const GenSet* gs = gen_set(b->mechset);
     std::vector<uint32_t> all;
-    int64_t pf_ctas = 0;  // the prefetch follows the members that hold most of the CTAs
     for (ngpu_sim* s : b->sims) {
         const std::vector<uint32_t> mm = model_masks(s->m);
         all.insert(all.end(), mm.begin(), mm.end());
-        pf_ctas += s->ch_prefetch ? s->n_groups : -s->n_groups;
     }
     const std::vector<uint32_t> picked = ngpu_jit::pick_masks(all, kMaxClasses);
     b->jit = ngpu_jit::module(b->mechset, b->precision == NGPU_FP64, picked, gs ? &gs->source : nullptr,
-                              pf_ctas >= 0, b->folds, masks_cover(picked, all, pf_ctas >= 0));
+                              b->folds, masks_cover(picked, all));
     if (gs && !b->jit)
         return fail(NGPU_E_CUDA, "mechanism set '" + gs->name +
                                      "' runs only through runtime compilation: " + ngpu_jit::last_log());

@@ -49,7 +49,6 @@ inline std::string float_literal(float v) {
 struct Module {
     int mechset = 0;
     bool fp64 = false;
-    bool prefetch = true;                   // channel-pass L2 prefetch compiled in (NGPU_CH_PREFETCH)
     bool complete = false;                  // the masks cover every node: no generic path (NGPU_CLASSES_COMPLETE)
     bool ti = false;                        // the thread-item layout's advance kernel compiled in
     int adv_warps = 8;                      // the advance kernels' CTA size bound (warps)
@@ -120,15 +119,14 @@ inline bool enabled() {
 // The generated translation unit: the init and advance kernels (single and
 // batch) over `masks`.  ms: the kernel template's mechanism set (0 TTPC,
 // 1 Mainen, 2 a generated set, whose channel code comes in as the extra
-// header ngpu_generated.cuh).  prefetch: the channel pass's L2 prefetch.
+// header ngpu_generated.cuh).
 // ti: also the thread-item layout's advance kernel.
 // adv_warps: the advance kernels are bounded for CTAs of up to this many
 // warps; above 8, for adv_ctas CTAs per SM (3 CTAs: 10 warps 64 registers,
 // 12: 56, 16: 40; 1 CTA, for batches of at most one CTA per SM: 16 warps
 // 128 registers).
-inline std::string source(int ms, bool fp64, const std::vector<uint32_t>& masks, bool prefetch = true,
-                          const Folds& folds = {}, bool complete = false, bool ti = false, int adv_warps = 8,
-                          int adv_ctas = 3) {
+inline std::string source(int ms, bool fp64, const std::vector<uint32_t>& masks, const Folds& folds = {},
+                          bool complete = false, bool ti = false, int adv_warps = 8, int adv_ctas = 3) {
     std::string list;
     for (size_t k = 0; k < masks.size(); ++k) list += (k ? ", " : "") + std::to_string(masks[k]) + "u";
     const std::string m = std::to_string(ms);
@@ -147,7 +145,6 @@ inline std::string source(int ms, bool fp64, const std::vector<uint32_t>& masks,
         fold += "}\n";
     }
     return std::string(ms == 2 ? "#define NGPU_GENERATED_NODE 1\n" : "") +
-           std::string(prefetch ? "" : "#define NGPU_CH_PREFETCH 0\n") +
            std::string(adv_warps > 8 && adv_ctas == 1 ? "#define NGPU_CH_AHEAD 0\n" : "") +
            std::string(complete ? "#define NGPU_CLASSES_COMPLETE 1\n" : "") + fold +
            "#include \"sim_kernels.cuh\"\n"
@@ -204,7 +201,7 @@ inline std::string cache_dir() {
 // through the on-disk cache.  Touches no device.  generated: the channel
 // code of a generated mechanism set (ms 2), or nullptr.
 inline bool build_cubin(int ms, bool fp64, const std::vector<uint32_t>& masks, const std::string* generated,
-                        const std::string& arch, std::vector<char>* out, std::string* err, bool prefetch = true,
+                        const std::string& arch, std::vector<char>* out, std::string* err,
                         const Folds& folds = {}, bool complete = false, bool ti = false, int adv_warps = 8,
                         int adv_ctas = 3) {
     const Nvrtc& nv = nvrtc();
@@ -212,7 +209,7 @@ inline bool build_cubin(int ms, bool fp64, const std::vector<uint32_t>& masks, c
         *err = last_log();
         return false;
     }
-    const std::string src = source(ms, fp64, masks, prefetch, folds, complete, ti, adv_warps, adv_ctas);
+    const std::string src = source(ms, fp64, masks, folds, complete, ti, adv_warps, adv_ctas);
     std::vector<std::string> opt_s = {"--gpu-architecture=sm_" + arch, "-std=c++17",
                                       "-lineinfo", "--ftz=true"};  // see ngpu_math.cuh
     int vmaj = 0, vmin = 0;
@@ -312,7 +309,7 @@ inline bool build_cubin(int ms, bool fp64, const std::vector<uint32_t>& masks, c
 // compilation is off or fails.  mechset >= 2 is a generated set whose channel
 // code is *generated.  Modules live until the process exits.
 inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>& masks,
-                            const std::string* generated, bool prefetch = true, const Folds& folds = {},
+                            const std::string* generated, const Folds& folds = {},
                             bool complete = false, bool ti = false, int adv_warps = 8, int adv_ctas = 3) {
     if (!generated && (!enabled() || masks.empty())) return nullptr;
     if (generated && !enabled()) {
@@ -321,7 +318,7 @@ inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>&
     }
     std::lock_guard<std::mutex> lock(mu());
     static std::map<std::string, std::unique_ptr<Module>> cache;
-    std::string key = std::to_string(mechset) + (fp64 ? "d" : "f") + (prefetch ? "p" : "n") + (complete ? "c" : "g") +
+    std::string key = std::to_string(mechset) + (fp64 ? "d" : "f") + (complete ? "c" : "g") +
                       (ti ? "t" : "") +
                       (adv_warps > 8 ? "w" + std::to_string(adv_warps) + "x" + std::to_string(adv_ctas) : std::string()) +
                       ":";
@@ -344,7 +341,7 @@ inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>&
     std::vector<char> cubin;
     std::string err;
     const std::string arch = std::to_string(maj) + std::to_string(min) + "a";
-    if (!build_cubin(generated ? 2 : mechset, fp64, masks, generated, arch, &cubin, &err, prefetch, folds,
+    if (!build_cubin(generated ? 2 : mechset, fp64, masks, generated, arch, &cubin, &err, folds,
                      complete, ti, adv_warps, adv_ctas)) {
         last_log() = err;
         cache[key] = nullptr;
@@ -353,7 +350,6 @@ inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>&
     auto mod = std::make_unique<Module>();
     mod->mechset = mechset;
     mod->fp64 = fp64;
-    mod->prefetch = prefetch;
     mod->complete = complete;
     mod->ti = ti;
     mod->adv_warps = adv_warps;

@@ -64,17 +64,9 @@ constexpr int kMaxWarps = 8;   // 256 threads; with 3 CTAs per SM the 85-registe
 #ifndef NGPU_ADV_MIN_BLOCKS
 #define NGPU_ADV_MIN_BLOCKS 3
 #endif
-// L2 prefetch of each node's state and parameter rows two nodes ahead in the
-// channel pass.  A compile-time choice: it pays on models whose nodes read
-// many rows (every node of the HH-type cells carries 7 mechanisms, ~30 rows)
-// and costs where most nodes read few (the TTPC-like cell, ~12), even when a
-// runtime flag turns it off; the runtime-specialised kernels set it per model.
-#ifndef NGPU_CH_PREFETCH
-#define NGPU_CH_PREFETCH 1
-#endif
-// Without that prefetch, the channel pass starts each node's loads one node
-// early (channels_item).  The runtime-specialised kernels for CTAs of more
-// than 8 warps at one CTA per SM turn it off: there it measured 4 % slower.
+// The channel pass starts each node's loads one node early (channels_item).
+// The runtime-specialised kernels for CTAs of more than 8 warps at one CTA
+// per SM turn it off: there it measured 4 % slower.
 #ifndef NGPU_CH_AHEAD
 #define NGPU_CH_AHEAD 1
 #endif
@@ -278,15 +270,6 @@ __device__ __forceinline__ void prefetch_backsub(const Group<R>& G, int i, int n
     if ((threadIdx.x & 31) == 0 && n > 0) {  // lane 0's pointers carry no lane offset
         prefetch_l2(G.scr + (size_t)i * 3 * kLanes, (uint32_t)n * 3 * kLanes * sizeof(R));
         prefetch_l2(G.vbuf + (size_t)i * 2 * kLanes, (uint32_t)n * 2 * kLanes * sizeof(R));
-    }
-}
-
-// L2 prefetch of the rows node n's channel update reads: states and parameters.
-template <typename R>
-__device__ __forceinline__ void prefetch_channels(const Group<R>& G, const NodeRec<R>& n) {
-    if ((threadIdx.x & 31) == 0) {
-        if (n.srows) prefetch_l2(G.slab + (size_t)n.srow * kLanes, n.srows * kLanes * sizeof(R));
-        if (n.prows) prefetch_l2(G.ptab + (size_t)n.prow * kLanes, n.prows * kLanes * sizeof(float));
     }
 }
 
@@ -700,17 +683,14 @@ __device__ __forceinline__ void channels_item(const SimArgs<R>& A, const Group<R
     SpineCarry<R> k;
     k.reset();
     R e_l = 0;
-    constexpr bool pf = NGPU_CH_PREFETCH != 0 && !TI;
-    // Without the bulk prefetch (models whose nodes read few rows), a node's
-    // loads are started one node early instead: its voltages (its own and
+    // A node's loads are started one node early: its voltages (its own and
     // its parent's; the pass writes no voltage) into registers, its state and
     // parameter rows into L2 (one prefetch per row, lane r taking row r).
     // Either alone measured slower on B200 (the node still waits for the
-    // other); both together, 2.7 % faster on the TTPC-like cell.  Models with
-    // the bulk prefetch keep the register budget for their channel code.
-    constexpr bool ahead = NGPU_CH_AHEAD != 0 && !pf && !TI;
-    if (pf && n > 0) prefetch_channels(G, nr[node_at(0)]);
-    if (pf && n > 1) prefetch_channels(G, nr[node_at(1)]);
+    // other); both together, 2.7 % faster on the TTPC-like cell.  (A bulk
+    // prefetch of the rows two nodes ahead paid on the HH cells while their
+    // channel code still branched; it costs 10 % since, at few instances.)
+    constexpr bool ahead = NGPU_CH_AHEAD != 0 && !TI;
     int vi = -1;  // node whose V was read last as a parent voltage (!ahead)
     R vv = 0;
     int i_nx = 0;  // the next node and its voltages (ahead)
@@ -723,7 +703,6 @@ __device__ __forceinline__ void channels_item(const SimArgs<R>& A, const Group<R
     for (int p = 0; p < n; ++p) {
         const int i = ahead ? i_nx : node_at(p);
         const NodeRec<R> nd = nr[i];
-        if (pf && p + 2 < n) prefetch_channels(G, nr[node_at(p + 2)]);
         R V, vp;
         if constexpr (ahead) {
             V = v_nx;
