@@ -184,8 +184,8 @@ int ngpu_sim_advance(ngpu_sim *s, int32_t t0, int32_t n_steps, void *cuda_stream
 int ngpu_sim_create_ex(ngpu_model *m, int32_t n_sets, int32_t n_stim, int32_t precision, int32_t n_warps,
                        ngpu_sim **out);
 /* As ngpu_sim_create_ex, also choosing how many work items per warp the tree
- * is split into (1..8; 0 = the library's choice: 2 where nodes read
- * many rows, 3 where they read few).  More items balance the warps'
+ * is split into (1..8; 0 = the library's choice: 3 for up to 8 warps, 1
+ * above).  More items balance the warps'
  * dynamic queue better at the price of more skeleton nodes; the best count
  * depends on the morphology, so the autotuner times it.  No counterpart in
  * the reference (one thread per compartment group, no split). */
@@ -197,7 +197,9 @@ int ngpu_sim_create_shaped(ngpu_model *m, int32_t n_sets, int32_t n_stim, int32_
  *       cta_warps warps sharing the tree (1..16; above 8 only through the
  *       runtime-compiled kernel, bounded for 3 CTAs per SM), items work
  *       items per warp (1..8); 0 = the library's choice.  With up to 8 warps
- *       this is ngpu_sim_create_shaped.
+ *       this is ngpu_sim_create_shaped.  Above 8 warps, a batch that leaves
+ *       SMs idle shares each group's tree between a cluster of up to 8 such
+ *       CTAs (one per SM).
  *       A B200 fills from about 148 x 32 x 2 instances on.
  *   NGPU_LAYOUT_WARP_INSTANCE  one warp per instance (its lanes share the
  *       instance's tree, split into `items` work items, 1..512; 0 = 32),

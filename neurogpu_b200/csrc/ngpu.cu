@@ -84,6 +84,11 @@ bool mechset_known(int ms) {
     return ms == NGPU_MECHSET_TTPC || ms == NGPU_MECHSET_MAINEN || gen_set(ms) != nullptr;
 }
 
+// A node's cost beside its mechanisms' (solve, voltage, row traffic), in the
+// units of MechDesc::cost: a passive node takes about half an HH node's time.
+// Weights that left it nearly out (12) gave one CTA of a team the TTPC-like
+// cell's 600 light basal nodes: 44.0 us per step at 300 instances, 33.4 with 80.
+constexpr int kNodeWeight = 80;
 const SetDesc& set_desc(int ms) {
     if (ms >= NGPU_MECHSET_GENERATED) return gen_set(ms)->desc;
     // TTPC: GUI/BBP_TTPC_EXAMPLE/pyNeuroGPU_unix/src/CudaStuff.cu:220 call list.
@@ -273,9 +278,16 @@ struct Partition {
     std::vector<int> sep_comp;      // segment component whose lower separator this is, or -1
     std::vector<int> jslot, pslot;
     int n_jslots = 0;
+    std::vector<int> skel;          // the staged skeleton's tables (SkelNode), by skeleton_tables
+    int n_lev = 0, n_chain_groups = 0, n_chains = 0;
 };
+// Shared memory of a lane-instance CTA over a split (staged: with the skeleton's staging rows).
+template <typename R>
+static size_t lane_smem(int n_nodes, const Partition& P, int staged) {
+    return staged ? SmemPlan<R>::bytes(n_nodes, (int)P.seps.size(), (int)P.skel.size()) : SmemPlan<R>::bytes(n_nodes);
+}
 
-static Partition make_partition(const ngpu_model* m, int W, int items_per_warp = 2) {
+static Partition make_partition_parts(const ngpu_model* m, int W, int64_t parts) {
     const int N = m->n;
     const std::vector<int>& par = m->parent;
     Partition P;
@@ -291,9 +303,7 @@ static Partition make_partition(const ngpu_model* m, int W, int items_per_warp =
         }
     }
     auto heavy = [&](int i) { return (i + 1 < N && par[i + 1] == i) ? i + 1 : -1; };
-    // items of at most ~1/(k W) of the cost: k items per warp balance the dynamic queue
-    // better than one, at a few more separators (the simulation chooses k per model)
-    const int64_t parts = W > 1 ? (int64_t)std::max(1, items_per_warp) * W : 1;
+    // items of at most ~1/parts of the cost
     const int64_t target = std::max<int64_t>(1, (subw[0] + parts - 1) / parts);
     std::vector<char> is_sep(N, 0);
     is_sep[0] = 1;
@@ -385,6 +395,86 @@ static Partition make_partition(const ngpu_model* m, int W, int items_per_warp =
     return P;
 }
 
+// W warps with k items each: more items balance the dynamic queue better, at
+// a few more separators.
+static Partition make_partition(const ngpu_model* m, int W, int items_per_warp = 2) {
+    return make_partition_parts(m, W, W > 1 ? (int64_t)std::max(1, items_per_warp) * W : 1);
+}
+
+// The staged skeleton's tables (SkelNode).
+static void skeleton_tables(Partition& P) {
+    const int S = (int)P.seps.size();
+    std::vector<std::vector<int>> kids(S);  // highest index first
+    std::vector<int> below(S, 1), heavy(S, -1), level(S, 0);
+    for (int k = S - 1; k > 0; --k) {  // a separator's skeleton parent comes before it
+        kids[P.sep_par[k]].push_back(k);
+        below[P.sep_par[k]] += below[k];
+    }
+    for (int k = 0; k < S; ++k)
+        for (int c : kids[k])
+            if (heavy[k] < 0 || below[c] > below[heavy[k]]) heavy[k] = c;
+    std::vector<int> heads;
+    for (int k = 0; k < S; ++k) {
+        const bool head = k == 0 || heavy[P.sep_par[k]] != k;
+        level[k] = k == 0 ? 0 : level[P.sep_par[k]] + (head ? 1 : 0);
+        if (head) heads.push_back(k);
+    }
+    auto up = [&](int h) { return P.sep_par[h]; };
+    std::stable_sort(heads.begin(), heads.end(),
+                     [&](int x, int y) { return level[x] != level[y] ? level[x] < level[y] : up(x) < up(y); });
+    const int levels = level[heads.back()] + 1;
+    std::vector<int> lev(levels + 1, 0), group, chain = {0}, order, place(S), par;
+    for (size_t c = 0; c < heads.size(); ++c) {
+        const int h = heads[c];
+        if (c == 0 || up(h) != up(heads[c - 1])) {
+            group.push_back((int)c);
+            lev[level[h] + 1]++;
+        }
+        std::vector<int> path;
+        for (int k = h; k >= 0; k = heavy[k]) path.push_back(k);
+        order.insert(order.end(), path.rbegin(), path.rend());
+        chain.push_back((int)order.size());
+    }
+    P.n_lev = levels;
+    P.n_chain_groups = (int)group.size();
+    P.n_chains = (int)heads.size();
+    group.push_back(P.n_chains);
+    for (int l = 0; l < levels; ++l) lev[l + 1] += lev[l];
+    for (int q = 0; q < S; ++q) place[order[q]] = q;
+    for (int h : heads) par.push_back(h ? place[up(h)] : -1);
+    std::vector<SkelNode> nd;
+    for (int k : order)
+        nd.push_back({(int16_t)k, (int16_t)P.seps[k], (int16_t)P.jslot[P.seps[k]], (int16_t)P.sep_comp[k]});
+    P.skel.clear();
+    for (const auto* v : {&lev, &group, &chain, &par}) P.skel.insert(P.skel.end(), v->begin(), v->end());
+    P.skel.resize(SmemPlan<float>::skel_ints(S, levels, P.n_chain_groups, P.n_chains), 0);
+    std::memcpy(P.skel.data() + SmemPlan<float>::skel_ofs(levels, P.n_chain_groups, P.n_chains), nd.data(),
+                sizeof(SkelNode) * nd.size());
+}
+
+// A team's work (SimArgs::team_items): items, and separators linked directly
+// to the skeleton, dealt to its CTAs largest first, each to the CTA with the
+// least so far.
+static std::vector<int> team_items(const ngpu_model* m, const Partition& P, int team) {
+    std::vector<std::pair<int64_t, int>> work;
+    const int C = (int)P.comps.size();
+    for (int k = 0; k < C; ++k) work.push_back({P.comps[k].weight, k});
+    for (int k = 0; k < (int)P.seps.size(); ++k)
+        if (P.sep_comp[k] < 0) work.push_back({m->weight[P.seps[k]], C + k});
+    std::stable_sort(work.begin(), work.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+    std::vector<std::vector<int>> mine(team);
+    std::vector<int64_t> load(team, 0);
+    for (const auto& x : work) {
+        const int c = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[c] += x.first;
+        mine[c].push_back(x.second);
+    }
+    std::vector<int> out = {0};
+    for (int c = 0; c < team; ++c) out.push_back(out.back() + (int)mine[c].size());
+    for (int c = 0; c < team; ++c) out.insert(out.end(), mine[c].begin(), mine[c].end());
+    return out;
+}
+
 struct ngpu_batch;
 struct ngpu_sim {
     ngpu_model* m = nullptr;
@@ -399,6 +489,9 @@ struct ngpu_sim {
     DevSep* d_seps = nullptr;
     void* d_sepv = nullptr;
     int n_warps = 1;
+    int team = 0;                 // CTAs (of n_warps warps) per group, one cluster; 0: one CTA per group
+    int* d_skel = nullptr;        // the staged skeleton's tables (part.skel)
+    int* d_team_items = nullptr;
     Partition part;
     double* d_jacc = nullptr;
     void* d_jx = nullptr;
@@ -429,7 +522,8 @@ struct ngpu_sim {
     const ngpu_jit::Module* jit = nullptr;
     ngpu_batch* batch = nullptr;  // the batch whose kernels this simulation's records follow
     int s2_stage = 0;             // skeleton solved from shared memory (see sim_kernels.cuh)
-    int items_per_warp = 2;       // work items per warp in the tree split
+    int items_per_warp = 3;       // work items per warp in the tree split
+    bool items_chosen = false;    // ... given by the caller
     ngpu_jit::Folds folds;        // parameters the runtime-specialised kernel compiles in
     uint2* d_prange = nullptr;    // [ptab_rows] bit-pattern range of each parameter row
     unsigned long long* d_phash = nullptr;  // [ptab_rows] hash of each parameter row
@@ -439,11 +533,13 @@ struct ngpu_sim {
     int ti_items = 32;            // thread-item layout: work items per instance's tree
 };
 
-// Rows (state and parameter) a node's channel update reads, on average, from
-// which on the tree is split into 2 items per warp instead of 3 (8-warp CTAs).
-// Measured on B200: the HH-type cells (~30 rows per node) run 9 % faster with
-// 2, the TTPC-like cell (~12) 5 % faster with 3.
-constexpr double kHeavyRowsPerNode = 20.0;
+// Work items per warp the tree is split into by default.  8-warp CTAs: 3
+// (ms per 200 steps at 12,288 instances with 1 / 2 / 3 / 4: TTPC-like 85.6 /
+// 83.6 / 77.6 / 83.3, HH 30.1 / 29.4 / 28.6 / 30.6).  Wide CTAs and teams: 1,
+// since a finer split lengthens the skeleton, which nothing hides there (us
+// per step with 1 / 2: HH cell, 33 instances 18.0 / 25.2; TTPC-like, 300
+// instances 33.4 / 40.6).
+static int default_items(int n_warps) { return n_warps > 8 ? 1 : 3; }
 
 // Thread-item layout: work items per instance at most / by default, and the
 // SM count the default CTA shape spreads a small batch over.
@@ -452,11 +548,10 @@ constexpr int kMaxTiItems = 512;
 // 3 CTAs per SM; the ahead-of-time kernels take up to kMaxWarps).
 constexpr int kMaxWideWarps = 16;
 constexpr int kDefaultTiItems = 32;
+// Compartments per warp of a wide CTA: a passive cable of 50 takes 8.7 us per
+// step with 6 warps, 6.4 with 16; one of 128, 20 with 4 and 9.4 with 16.
+constexpr int kWideNodes = 3;
 constexpr int kSmCount = 148;
-
-static double rows_per_node(const ngpu_model* m) {
-    return m->n > 0 ? (double)(m->state_vars + m->param_reads) / m->n : 0.0;
-}
 
 // CTAs per SM that `smem` bytes of dynamic shared memory and W warps of 80
 // registers allow (228 KB per SM, 1 KB of it reserved per CTA).
@@ -464,6 +559,53 @@ static double rows_per_node(const ngpu_model* m) {
 // for: 1 when the batch has at most one group per SM (registers are then
 // plentiful: 16 warps get 128), else 3 (one wave for large batches).
 static int wide_ctas_per_sm(int n_groups) { return n_groups <= kSmCount ? 1 : 3; }
+
+__global__ void k_cluster_probe() {}  // never launched: its occupancy is asked for
+
+// Clusters of `size` CTAs, one CTA per SM, that the device runs at once (its
+// SMs come in uneven clusters of their own, so this is not SMs / size).
+static int max_clusters(int size) {
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, int> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find({dev, size});
+    if (it != known.end()) return it->second;
+    const int smem = 120 * 1024;  // one CTA per SM
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)size;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)size * 148);
+    cfg.blockDim = dim3(kLanes * kMaxWarps);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const void* k = (const void*)k_cluster_probe;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return known[{dev, size}] = n;
+}
+
+// CTAs (one per SM, a cluster) that share a group's tree: as many as run at
+// once for every group, up to one per kTeamNodes compartments.  Measured on
+// B200 (us per step): HH cell of 500, 33 instances: 1 CTA 42, 4 20.7, 6 18.8,
+// 8 19.6 (the skeleton grows with the CTAs); TTPC-like cell of 1501, 300
+// instances: 1 CTA 108, 4 63.9, 8 43.5; HH cell in FP64, 768 instances: 1 CTA
+// 161, 5 51.5, 6 (more clusters than run at once) 84.4; passive cable of 128:
+// 1 CTA 9.4, 2 9.6.
+constexpr int kTeamNodes = 80;
+static int team_size(int n_groups, int n_nodes) {
+    for (int c = std::min(8, n_nodes / kTeamNodes); c > 1; --c)
+        if (n_groups <= max_clusters(c)) return c;
+    return 0;
+}
 
 static int ctas_per_sm(size_t smem, int W, int n_groups) {
     // kernels of up to 8 warps use 80 registers; wider ones are compiled for wide_ctas_per_sm
@@ -474,9 +616,9 @@ static int ctas_per_sm(size_t smem, int W, int n_groups) {
 
 // Stage the skeleton in shared memory when that costs no occupancy.
 template <typename R>
-static int choose_s2_stage(int n_nodes, int n_seps, int W, int n_groups) {
-    if (W < 2 || n_seps < 2) return 0;
-    const size_t plain = SmemPlan<R>::bytes(n_nodes), staged = SmemPlan<R>::bytes(n_nodes, n_seps, 1);
+static int choose_s2_stage(int n_nodes, const Partition& P, int W, int n_groups) {
+    if (W < 2 || P.seps.size() < 2) return 0;
+    const size_t plain = lane_smem<R>(n_nodes, P, 0), staged = lane_smem<R>(n_nodes, P, 1);
     return staged <= 227 * 1024 && ctas_per_sm(staged, W, n_groups) >= ctas_per_sm(plain, W, n_groups) ? 1 : 0;
 }
 
@@ -515,6 +657,12 @@ static SimArgs<R> make_args(ngpu_sim* s) {
     A.n_seps = (int)s->part.seps.size();
     A.sepv = (R*)s->d_sepv;
     A.s2_stage = s->s2_stage;
+    A.skel = s->d_skel;
+    A.n_lev = s->part.n_lev;
+    A.n_groups = s->part.n_chain_groups;
+    A.n_chains = s->part.n_chains;
+    A.team = s->team;
+    A.team_items = s->d_team_items;
     return A;
 }
 
@@ -560,14 +708,29 @@ static cudaError_t launch_advance(ngpu_sim* s, int t0, int n, cudaStream_t st) {
     if (s->layout == NGPU_LAYOUT_WARP_INSTANCE) return launch_advance_ti<R>(s, t0, n, st);
     SimArgs<R> A = make_args<R>(s);
     const int threads = kLanes * s->n_warps;
-    const size_t smem = SmemPlan<R>::bytes(s->m->n, (int)s->part.seps.size(), s->s2_stage);
+    const size_t smem = lane_smem<R>(s->m->n, s->part, s->s2_stage);
     cudaError_t e;
     if (s->jit) {
         const void* k = (const void*)s->jit->advance;
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         void* args[] = {(void*)&A, (void*)&t0, (void*)&n};
-        e = cudaLaunchKernel(k, dim3(s->n_groups), dim3(threads), args, smem, st);
+        if (s->team) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = (unsigned)s->team;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3((unsigned)(s->n_groups * s->team));
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            e = cudaLaunchKernelExC(&cfg, k, args);
+        } else {
+            e = cudaLaunchKernel(k, dim3(s->n_groups), dim3(threads), args, smem, st);
+        }
         g_launches++;
         return e != cudaSuccess ? e : cudaGetLastError();
     }
@@ -710,7 +873,7 @@ int ngpu_model_create(int32_t n_nodes, const int32_t* parent, const double* a, c
     // recording nodes are mapped through the permutation.
     std::vector<int64_t> subw(n_nodes, 0);
     for (int i = n_nodes - 1; i >= 0; --i) {
-        int wt = 12;
+        int wt = kNodeWeight;
         for (int k = 0; k < NM; ++k)
             if (mask0[i] & (1u << k)) wt += sd.mechs[k].cost;
         subw[i] += wt;
@@ -783,7 +946,7 @@ int ngpu_model_create(int32_t n_nodes, const int32_t* parent, const double* a, c
         ni.parent = m->parent[i];
         ni.mask = m->mask[i];
         ni.srow = srow;
-        int srows = 0, wt = 12;
+        int srows = 0, wt = kNodeWeight;
         std::vector<int> plist;
         for (int k = 0; k < NM; ++k)
             if (ni.mask & (1u << k)) {
@@ -924,7 +1087,7 @@ static void sim_free(ngpu_sim* s) {
     void* ptrs[] = {s->d_nodes, s->d_vbuf, s->d_slab, s->d_ptab, s->d_scr, s->d_jacc, s->d_jx,
                     s->d_inst_stim, s->d_bad, s->d_row_param, s->d_row_sec, s->d_amps,
                     s->d_dts, s->d_trace, s->d_tmp_out, s->d_comps, s->d_seps, s->d_sepv, s->d_prange,
-                    s->d_phash, s->d_params_in};
+                    s->d_phash, s->d_params_in, s->d_skel, s->d_team_items};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (s->h_stage) cudaFreeHost(s->h_stage);
@@ -973,11 +1136,36 @@ static void host_copy_parallel(void* dst, const void* src, size_t bytes) {
     for (auto& t : th) t.join();
 }
 
+// The tree split of a lane-instance simulation for its n_warps, items_per_warp
+// and batch size.
+static void sim_split_lanes(ngpu_sim* s) {
+    const ngpu_model* m = s->m;
+    const bool f8 = s->precision == NGPU_FP64;
+    s->team = 0;
+    int team = s->n_warps > kMaxWarps ? team_size(s->n_groups, m->n) : 0;
+    if (const char* ev = getenv("NGPU_TEAM")) team = std::min(team, atoi(ev));
+    for (; team > 1; --team) {
+        s->part = make_partition(m, s->n_warps * team, s->items_per_warp);
+        skeleton_tables(s->part);
+        const size_t smem = f8 ? lane_smem<double>(m->n, s->part, 1) : lane_smem<float>(m->n, s->part, 1);
+        if (smem <= 227 * 1024 - 64 && s->part.seps.size() > 1) {
+            s->team = team;
+            s->s2_stage = 1;
+            return;
+        }
+    }
+    s->part = make_partition(m, s->n_warps, s->items_per_warp);
+    skeleton_tables(s->part);
+    s->s2_stage = f8 ? choose_s2_stage<double>(m->n, s->part, s->n_warps, s->n_groups)
+                     : choose_s2_stage<float>(m->n, s->part, s->n_warps, s->n_groups);
+}
+
 // The device side of the simulation's tree split (s->part): junction
 // accumulators and dV slots, work items, separators and segment links,
 // (re)allocated for the split and its items and separators uploaded.
 static int sim_upload_split(ngpu_sim* s) {
-    void** old[] = {(void**)&s->d_jacc, (void**)&s->d_jx, (void**)&s->d_comps, (void**)&s->d_seps, &s->d_sepv};
+    void** old[] = {(void**)&s->d_jacc, (void**)&s->d_jx, (void**)&s->d_comps, (void**)&s->d_seps, &s->d_sepv,
+                    (void**)&s->d_skel, (void**)&s->d_team_items};
     for (void** p : old)
         if (*p) {
             cudaFree(*p);
@@ -986,11 +1174,12 @@ static int sim_upload_split(ngpu_sim* s) {
     const size_t G = (size_t)s->n_groups, L = kLanes, esz = s->precision == NGPU_FP64 ? 8 : 4;
     const size_t nj = std::max(1, s->part.n_jslots), ns = std::max<size_t>(1, s->part.seps.size());
     int rc = NGPU_OK;
-    if (!(s->d_jacc = (double*)dmalloc(G * 2 * nj * L * sizeof(double), &rc))) return rc;
+    const size_t copies = s->team ? 3 : 1, links = s->team ? kTeamRows : 4;  // see advance_body
+    if (!(s->d_jacc = (double*)dmalloc(copies * G * 2 * nj * L * sizeof(double), &rc))) return rc;
     if (!(s->d_jx = dmalloc(G * nj * L * esz, &rc))) return rc;
     if (!(s->d_comps = (DevComp*)dmalloc(sizeof(DevComp) * std::max<size_t>(1, s->part.comps.size()), &rc))) return rc;
     if (!(s->d_seps = (DevSep*)dmalloc(sizeof(DevSep) * ns, &rc))) return rc;
-    if (!(s->d_sepv = dmalloc(G * 4 * ns * L * esz, &rc))) return rc;
+    if (!(s->d_sepv = dmalloc(copies * G * links * ns * L * esz, &rc))) return rc;
     std::vector<DevComp> dc;
     for (const Comp& c : s->part.comps) dc.push_back({c.r, c.u, c.l, c.lk, c.light_lo, c.light_hi});
     std::vector<DevSep> ds;
@@ -998,6 +1187,15 @@ static int sim_upload_split(ngpu_sim* s) {
         ds.push_back({s->part.seps[k], s->part.sep_par[k], s->part.sep_comp[k], 0});
     if (!dc.empty()) NGPU_CUDA(cudaMemcpy(s->d_comps, dc.data(), sizeof(DevComp) * dc.size(), cudaMemcpyHostToDevice));
     NGPU_CUDA(cudaMemcpy(s->d_seps, ds.data(), sizeof(DevSep) * ds.size(), cudaMemcpyHostToDevice));
+    if (!s->part.skel.empty()) {
+        if (!(s->d_skel = (int*)dmalloc(sizeof(int) * s->part.skel.size(), &rc))) return rc;
+        NGPU_CUDA(cudaMemcpy(s->d_skel, s->part.skel.data(), sizeof(int) * s->part.skel.size(), cudaMemcpyHostToDevice));
+    }
+    if (s->team) {
+        const std::vector<int> ti = team_items(s->m, s->part, s->team);
+        if (!(s->d_team_items = (int*)dmalloc(sizeof(int) * ti.size(), &rc))) return rc;
+        NGPU_CUDA(cudaMemcpy(s->d_team_items, ti.data(), sizeof(int) * ti.size(), cudaMemcpyHostToDevice));
+    }
     return NGPU_OK;
 }
 
@@ -1056,22 +1254,22 @@ int ngpu_sim_create_layout(ngpu_model* m, int32_t n_sets, int32_t n_stim, int32_
     const size_t esz = precision == NGPU_FP64 ? 8 : 4;
     const size_t G = (size_t)s->n_groups, L = kLanes;
     int rc = NGPU_OK;
-    // warps per CTA and the tree split over them
-    // warps per CTA: a batch of at most one 32-instance group per SM leaves SMs
-    // idle, so its CTAs get up to 16 warps (a finer split of the tree, the
-    // runtime-compiled kernel at one CTA per SM: the HH cell at 2457
-    // instances runs 1.4x faster, the TTPC-like cell at 33 instances 1.5x);
-    // larger batches up to 8 (three CTAs per SM at 80 registers)
+    // warps per CTA and the tree split over them: a batch of at most one
+    // 32-instance group per SM leaves SMs idle, so its CTAs get up to 16 warps
+    // at one CTA per SM, and where SMs are still left a group gets a team of
+    // CTAs (sim_split_lanes); larger batches up to 8 (three CTAs per SM at 80
+    // registers)
     int W = std::min(8, std::max(1, m->n / 48));
     if (s->n_groups <= kSmCount && !ti && ngpu_jit::enabled() && ngpu_jit::nvrtc().ok)
-        W = std::min(kMaxWideWarps, std::max(1, m->n / 32));
+        W = std::min(kMaxWideWarps, std::max(1, m->n / kWideNodes));
     if (const char* ev = getenv("NGPU_WARPS")) W = std::max(1, std::min(kMaxWideWarps, atoi(ev)));
     if (n_warps > 0) W = n_warps;
     W = std::min(W, m->n);
     s->n_warps = W;
-    s->items_per_warp = rows_per_node(m) >= kHeavyRowsPerNode ? 2 : 3;
+    s->items_per_warp = default_items(W);
     if (const char* ev = getenv("NGPU_ITEMS_PER_WARP")) s->items_per_warp = std::max(1, std::min(8, atoi(ev)));
     if (items_per_warp > 0) s->items_per_warp = items_per_warp;
+    s->items_chosen = items_per_warp > 0;
     if (ti) {
         // one warp per instance: the tree split into ti_items items for the
         // warp's lanes; CTAs of ti_warps instances, enough CTAs for every SM
@@ -1093,9 +1291,7 @@ int ngpu_sim_create_layout(ngpu_model* m, int32_t n_sets, int32_t n_stim, int32_
                                             " bytes of shared memory per CTA; use fewer instances per CTA or items");
         }
     } else {
-        s->part = make_partition(m, W, s->items_per_warp);
-        s->s2_stage = precision == NGPU_FP64 ? choose_s2_stage<double>(m->n, (int)s->part.seps.size(), W, s->n_groups)
-                                             : choose_s2_stage<float>(m->n, (int)s->part.seps.size(), W, s->n_groups);
+        sim_split_lanes(s);
     }
 #define ALLOC(field, type, bytes)                              \
     s->field = (type)dmalloc((bytes), &rc);                    \
@@ -1512,7 +1708,7 @@ static int sim_upload_nodes(ngpu_sim* s) {
                                       s->folds, masks_cover(picked, all),
                                       s->layout == NGPU_LAYOUT_WARP_INSTANCE,
                                       s->layout == NGPU_LAYOUT_LANE_INSTANCE ? std::max(8, s->n_warps) : 8,
-                                      wide_ctas_per_sm(s->n_groups));
+                                      wide_ctas_per_sm(s->n_groups), s->team != 0);
         }
         if (gs && !s->jit)
             return fail(NGPU_E_CUDA, "mechanism set '" + gs->name +
@@ -1681,10 +1877,8 @@ int ngpu_batch_create(ngpu_sim* const* sims, int32_t n, ngpu_batch** out) {
         if (s->n_warps <= kMaxWarps) continue;
         const int W = std::min(kMaxWarps, std::max(1, s->m->n / 48));
         s->n_warps = W;
-        s->part = make_partition(s->m, W, s->items_per_warp);
-        s->s2_stage = s->precision == NGPU_FP64
-                          ? choose_s2_stage<double>(s->m->n, (int)s->part.seps.size(), W, s->n_groups)
-                          : choose_s2_stage<float>(s->m->n, (int)s->part.seps.size(), W, s->n_groups);
+        if (!s->items_chosen) s->items_per_warp = default_items(W);
+        sim_split_lanes(s);
         const int rc = sim_upload_split(s);
         if (rc != NGPU_OK) return rc;
         s->initialized = false;
@@ -1698,9 +1892,8 @@ int ngpu_batch_create(ngpu_sim* const* sims, int32_t n, ngpu_batch** out) {
     for (ngpu_sim* s : b->sims) {
         W = std::max(W, s->n_warps);
         b->total_ctas += s->n_groups;
-        const int ns = (int)s->part.seps.size();
-        b->smem = std::max(b->smem, b->precision == NGPU_FP64 ? SmemPlan<double>::bytes(s->m->n, ns, s->s2_stage)
-                                                             : SmemPlan<float>::bytes(s->m->n, ns, s->s2_stage));
+        b->smem = std::max(b->smem, b->precision == NGPU_FP64 ? lane_smem<double>(s->m->n, s->part, s->s2_stage)
+                                                             : lane_smem<float>(s->m->n, s->part, s->s2_stage));
     }
     b->threads = kLanes * W;
     b->folds = batch_common_folds(b);
@@ -2337,6 +2530,10 @@ extern "C" int ngpu_run_static(ngpu_model* m, int32_t n_sets, const float* param
     A.n_seps = 1;
     A.sepv = (float*)(base + o_sepv);
     A.s2_stage = 0;
+    A.skel = nullptr;
+    A.n_lev = A.n_groups = A.n_chains = 0;
+    A.team = 0;
+    A.team_items = nullptr;
 
     const size_t total = G * m->ptab_rows * L;
     const int blocks = (int)std::min<size_t>((total + 255) / 256, 148 * 16);

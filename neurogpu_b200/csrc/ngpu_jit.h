@@ -53,6 +53,7 @@ struct Module {
     bool ti = false;                        // the thread-item layout's advance kernel compiled in
     int adv_warps = 8;                      // the advance kernels' CTA size bound (warps)
     int adv_ctas = 3;                       // ... and CTAs per SM they are compiled for (above 8 warps)
+    bool team = false;                      // the advance kernel runs a cluster of CTAs per group
     std::vector<uint32_t> masks;            // class k runs the code for masks[k]
     cudaLibrary_t lib = nullptr;
     cudaKernel_t init = nullptr;           // (SimArgs<R>)
@@ -121,12 +122,13 @@ inline bool enabled() {
 // 1 Mainen, 2 a generated set, whose channel code comes in as the extra
 // header ngpu_generated.cuh).
 // ti: also the thread-item layout's advance kernel.
+// team: the advance kernel is the one for clusters of CTAs (advance_body).
 // adv_warps: the advance kernels are bounded for CTAs of up to this many
 // warps; above 8, for adv_ctas CTAs per SM (3 CTAs: 10 warps 64 registers,
 // 12: 56, 16: 40; 1 CTA, for batches of at most one CTA per SM: 16 warps
 // 128 registers).
 inline std::string source(int ms, bool fp64, const std::vector<uint32_t>& masks, const Folds& folds = {},
-                          bool complete = false, bool ti = false, int adv_warps = 8, int adv_ctas = 3) {
+                          bool complete = false, bool ti = false, int adv_warps = 8, int adv_ctas = 3, bool team = false) {
     std::string list;
     for (size_t k = 0; k < masks.size(); ++k) list += (k ? ", " : "") + std::to_string(masks[k]) + "u";
     const std::string m = std::to_string(ms);
@@ -158,7 +160,8 @@ inline std::string source(int ms, bool fp64, const std::vector<uint32_t>& masks,
            "ngpu_jit_advance(ngpu::SimArgs<" + R + "> A, int t0, int n_steps) {\n"
            "    extern __shared__ __align__(128) char smem[];\n"
            "    __shared__ int ctr[2];\n"
-           "    ngpu::advance_body<" + R + ", " + m + ", JitClasses>(A, blockIdx.x, t0, n_steps, smem, ctr);\n"
+           "    ngpu::advance_body<" + R + ", " + m + ", JitClasses" +
+           (team ? ", true>(A, blockIdx.x / A.team" : ">(A, blockIdx.x") + ", t0, n_steps, smem, ctr);\n"
            "}\n"
            "extern \"C\" __global__ void __launch_bounds__(ngpu::kLanes * ngpu::kMaxWarps)\n"
            "ngpu_jit_batch_init(const __grid_constant__ ngpu::BatchArgs<" + R + "> B) {\n"
@@ -203,13 +206,13 @@ inline std::string cache_dir() {
 inline bool build_cubin(int ms, bool fp64, const std::vector<uint32_t>& masks, const std::string* generated,
                         const std::string& arch, std::vector<char>* out, std::string* err,
                         const Folds& folds = {}, bool complete = false, bool ti = false, int adv_warps = 8,
-                        int adv_ctas = 3) {
+                        int adv_ctas = 3, bool team = false) {
     const Nvrtc& nv = nvrtc();
     if (!nv.ok) {
         *err = last_log();
         return false;
     }
-    const std::string src = source(ms, fp64, masks, folds, complete, ti, adv_warps, adv_ctas);
+    const std::string src = source(ms, fp64, masks, folds, complete, ti, adv_warps, adv_ctas, team);
     std::vector<std::string> opt_s = {"--gpu-architecture=sm_" + arch, "-std=c++17",
                                       "-lineinfo", "--ftz=true"};  // see ngpu_math.cuh
     int vmaj = 0, vmin = 0;
@@ -310,7 +313,8 @@ inline bool build_cubin(int ms, bool fp64, const std::vector<uint32_t>& masks, c
 // code is *generated.  Modules live until the process exits.
 inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>& masks,
                             const std::string* generated, const Folds& folds = {},
-                            bool complete = false, bool ti = false, int adv_warps = 8, int adv_ctas = 3) {
+                            bool complete = false, bool ti = false, int adv_warps = 8, int adv_ctas = 3,
+                            bool team = false) {
     if (!generated && (!enabled() || masks.empty())) return nullptr;
     if (generated && !enabled()) {
         last_log() = "runtime compilation is off (NGPU_JIT=0)";
@@ -319,7 +323,7 @@ inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>&
     std::lock_guard<std::mutex> lock(mu());
     static std::map<std::string, std::unique_ptr<Module>> cache;
     std::string key = std::to_string(mechset) + (fp64 ? "d" : "f") + (complete ? "c" : "g") +
-                      (ti ? "t" : "") +
+                      (ti ? "t" : "") + (team ? "m" : "") +
                       (adv_warps > 8 ? "w" + std::to_string(adv_warps) + "x" + std::to_string(adv_ctas) : std::string()) +
                       ":";
     for (uint32_t m : masks) key += std::to_string(m) + ",";
@@ -342,7 +346,7 @@ inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>&
     std::string err;
     const std::string arch = std::to_string(maj) + std::to_string(min) + "a";
     if (!build_cubin(generated ? 2 : mechset, fp64, masks, generated, arch, &cubin, &err, folds,
-                     complete, ti, adv_warps, adv_ctas)) {
+                     complete, ti, adv_warps, adv_ctas, team)) {
         last_log() = err;
         cache[key] = nullptr;
         return nullptr;
@@ -354,6 +358,7 @@ inline const Module* module(int mechset, bool fp64, const std::vector<uint32_t>&
     mod->ti = ti;
     mod->adv_warps = adv_warps;
     mod->adv_ctas = adv_ctas;
+    mod->team = team;
     mod->masks = masks;
     cudaError_t e = cudaLibraryLoadData(&mod->lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->init, mod->lib, "ngpu_jit_init");

@@ -60,6 +60,7 @@
 namespace ngpu {
 
 constexpr int kLanes = 32;
+constexpr int kTeamRows = 7;   // rows a team exchanges per separator: the segment link's 4, the assembled row's 3
 constexpr int kMaxWarps = 8;   // 256 threads; with 3 CTAs per SM the 85-register cap keeps a whole batch resident
 #ifndef NGPU_ADV_MIN_BLOCKS
 #define NGPU_ADV_MIN_BLOCKS 3
@@ -103,6 +104,18 @@ struct DevComp {
 struct DevSep {
     int node, par, seg, pad;
 };
+// The skeleton as its staged solve walks it.  Its heavy paths (each node
+// with its child of most separators below it) are chains, a chain's level
+// the number of chains above it: a few levels even for a skeleton that is
+// one long path.  A level's chains that end at the same parent form a group,
+// walked by one warp.  The tables (SimArgs::skel) hold the level offsets
+// into the groups, the group offsets into the chains, the chain offsets into
+// the nodes, the place of each chain's parent, and the nodes chain by chain,
+// from bottom to head; a node's place in that list is also its row in the
+// staging arrays.
+struct alignas(8) SkelNode {
+    int16_t k, node, jslot, seg;  // separator index, tree node, junction slot, linking segment or -1
+};
 
 template <typename R>
 struct SimArgs {
@@ -137,6 +150,11 @@ struct SimArgs {
     int n_seps;
     R* sepv;               // [n_seps][4] rows per group: A, B, excess, rhs terms of segment links
     int s2_stage;          // skeleton solve from shared memory (SmemPlan)
+    const int* skel;       // the staged skeleton's tables (SkelNode)
+    int n_lev, n_groups, n_chains;
+    // a team of CTAs (one cluster) per group; see advance_body
+    int team;              // CTAs per group (0: one, and none of the rest is set)
+    const int* team_items; // [team + 1] offsets, then the work items of each CTA, by decreasing cost
 };
 
 // mk: the node's mechanism bits, a runtime value or a std::integral_constant
@@ -239,14 +257,24 @@ __device__ __forceinline__ Group<R> group_of(const SimArgs<R>& A, int g) {
 // Shared memory: the node records, then (s2_stage) the skeleton's staging
 // rows, [n_seps][32] each: two FP64 accumulators (excess, right-hand side)
 // and five R rows (coupling A / later c, coupling B / later r, axial term
-// e / later dV, V, Kahan term).
+// e / later dV, V, Kahan term), and the skeleton's tables.
 template <typename R>
 struct SmemPlan {
     static __host__ __device__ size_t nodes(int n_nodes) {
         return (sizeof(NodeRec<R>) * (size_t)n_nodes + 15) / 16 * 16;
     }
-    static __host__ __device__ size_t bytes(int n_nodes, int n_seps = 0, int stage = 0) {
-        return nodes(n_nodes) + (stage ? (size_t)n_seps * 32 * (2 * sizeof(double) + 5 * sizeof(R)) : 0);
+    // the skeleton's tables: level, group and chain offsets, parents, nodes
+    static __host__ __device__ int skel_ofs(int n_lev, int n_groups, int n_chains) {
+        return (n_lev + n_groups + 2 * n_chains + 3 + 1) / 2 * 2;
+    }
+    static __host__ __device__ int skel_ints(int n_seps, int n_lev, int n_groups, int n_chains) {
+        return skel_ofs(n_lev, n_groups, n_chains) + n_seps * (int)(sizeof(SkelNode) / 4);
+    }
+    // the staged skeleton: per separator two FP64 rows and five R rows, and the tables
+    static __host__ __device__ size_t bytes(int n_nodes, int n_seps = 0, int skel_words = 0) {
+        return nodes(n_nodes) + (skel_words ? (size_t)n_seps * 32 * (2 * sizeof(double) + 5 * sizeof(R)) +
+                                                  ((size_t)skel_words * 4 + 15) / 16 * 16
+                                            : 0);
     }
     // thread-item layout: the node records, then per warp (one instance) the
     // skeleton's staging rows, [n_seps] each of the same seven
@@ -370,11 +398,14 @@ __device__ __forceinline__ void assemble_node(const SimArgs<R>& A, const Group<R
 }
 
 template <typename R>
-__device__ __forceinline__ void store_row(const Group<R>& G, int i, R x, R rhs, R e) {
-    R* o = G.scr + (size_t)i * 3 * kLanes;
+__device__ __forceinline__ void store_row_at(R* o, R x, R rhs, R e) {
     o[0] = x;
     o[kLanes] = rhs;
     o[2 * kLanes] = e;
+}
+template <typename R>
+__device__ __forceinline__ void store_row(const Group<R>& G, int i, R x, R rhs, R e) {
+    store_row_at(G.scr + (size_t)i * 3 * kLanes, x, rhs, e);
 }
 
 template <typename R>
@@ -423,6 +454,35 @@ __device__ __forceinline__ const NodeRec<R>* stage_nodes(const SimArgs<R>& A, ch
     __syncthreads();
     return nr;
 }
+
+// The staged skeleton's shared-memory rows and tables (SmemPlan).
+template <typename R>
+struct Skel {
+    double *acx, *acr;
+    R *sA, *sB, *sE, *sV, *sC;
+    const int *lev, *group, *chain, *par;
+    const SkelNode* nd;
+    __device__ __forceinline__ Skel(const SimArgs<R>& A, char* smem) {
+        const size_t row = (size_t)A.n_seps * kLanes;
+        acx = (double*)(smem + SmemPlan<R>::nodes(A.n_nodes));
+        acr = acx + row;
+        sA = (R*)(acr + row);
+        sB = sA + row;
+        sE = sB + row;
+        sV = sE + row;
+        sC = sV + row;
+        lev = (const int*)(sC + row);
+        group = lev + A.n_lev + 1;
+        chain = group + A.n_groups + 1;
+        par = chain + A.n_chains + 1;
+        nd = (const SkelNode*)(lev + SmemPlan<R>::skel_ofs(A.n_lev, A.n_groups, A.n_chains));
+    }
+    __device__ __forceinline__ void load_tables(const SimArgs<R>& A) const {
+        int* t = const_cast<int*>(lev);
+        const int n = SmemPlan<R>::skel_ints(A.n_seps, A.n_lev, A.n_groups, A.n_chains);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) t[i] = A.skel[i];
+    }
+};
 
 // Segment item, leaf -> root elimination of the spine r..l-1 (after its
 // light subtrees).  Each spine row also couples to the lower separator's dV
@@ -494,12 +554,12 @@ __device__ __forceinline__ void eliminate_spine_row(const Group<R>& G, const Nod
 
 // The spine of segment c, from rows supplied by row(i, x, rhs, e).
 template <typename R, typename Row>
-__device__ __forceinline__ void eliminate_segment(const Group<R>& G, const NodeRec<R>* nr, const DevComp& c, R e_l,
-                                                  Row&& row) {
+__device__ __forceinline__ void eliminate_segment(const Group<R>& G, const NodeRec<R>* nr, const DevComp& c, int link,
+                                                  R e_l, Row&& row) {
     const NodeRec<R> nl = nr[c.l];
     SpineCarry<R> k;
     k.reset();
-    R* sv = G.sepv + (size_t)c.lk * 4 * kLanes;
+    R* sv = G.sepv + (size_t)(c.lk * link) * kLanes;  // link: rows per separator
     for (int i = c.l - 1; i >= c.r; --i) {
         R x0, r0, e_i;
         row(i, x0, r0, e_i);
@@ -524,8 +584,15 @@ __device__ __forceinline__ void init_body(const SimArgs<R>& A, int g, int* ctr) 
     const Group<R> G = group_of(A, g);
     const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (threadIdx.x == 0) *ctr = 0;
+    Group<R> H = G;  // where the items' links and accumulators go: a team's first copy
+    int link = 4;
+    if (A.team) {
+        H.jacc = A.jacc + (size_t)g * 6 * A.n_jslots * kLanes + (threadIdx.x & 31);
+        H.sepv = A.sepv + (size_t)g * 3 * kTeamRows * A.n_seps * kLanes + (threadIdx.x & 31);
+        link = kTeamRows;
+    }
     if (w == 0)
-        for (int j = 0; j < 2 * A.n_jslots; ++j) G.jacc[(size_t)j * kLanes] = 0.0;
+        for (int j = 0; j < (A.team ? 6 : 2) * A.n_jslots; ++j) H.jacc[(size_t)j * kLanes] = 0.0;
     R dt, dtn_inv, istim_amp;
     bool rec_now;
     float* trace;
@@ -551,9 +618,14 @@ __device__ __forceinline__ void init_body(const SimArgs<R>& A, int g, int* ctr) 
     };
     for (int k = next_item(ctr); k < A.n_comps; k = next_item(ctr)) {
         const DevComp c = A.comps[k];
-        eliminate_range(G, A.nodes, c.lo, c.hi, row);
-        if (c.l >= 0) eliminate_segment(G, A.nodes, c, G.scr[(size_t)c.l * 3 * kLanes + 2 * kLanes], row);
+        eliminate_range(H, A.nodes, c.lo, c.hi, row);
+        if (c.l >= 0) eliminate_segment(H, A.nodes, c, link, G.scr[(size_t)c.l * 3 * kLanes + 2 * kLanes], row);
     }
+    if (A.team)  // the separators' assembled rows (read above, never eliminated by an item)
+        for (int k = w; k < A.n_seps; k += nw) {
+            const R* o = G.scr + (size_t)A.seps[k].node * 3 * kLanes;
+            store_row_at(H.sepv + (size_t)(k * kTeamRows + 4) * kLanes, o[0], o[kLanes], o[2 * kLanes]);
+        }
 }
 
 template <typename R, int MS>
@@ -665,9 +737,9 @@ __device__ __forceinline__ void backsub_item(const SimArgs<R>& A, const Group<R>
 // skeleton: its row goes to the skeleton), and, for a segment (lk >= 0),
 // the spine sep-1 .. r.  Every channel update of a step goes through this
 // one loop, so the channel code is inlined once.
-template <typename R, int MS, typename Classes, bool TI = false>
+template <typename R, int MS, typename Classes, bool TI = false, bool TEAM = false>
 __device__ __forceinline__ void channels_item(const SimArgs<R>& A, const Group<R>& G, const NodeRec<R>* nr,
-                                              int lo, int hi, int sep, int r, int lk, R dt, R dtn_inv,
+                                              int lo, int hi, int sep, int sepk, int r, int lk, R dt, R dtn_inv,
                                               R istim_amp) {
     const int n_light = hi - lo;
     const int n_sep = n_light + (sep >= 0 ? 1 : 0);
@@ -678,7 +750,7 @@ __device__ __forceinline__ void channels_item(const SimArgs<R>& A, const Group<R
     R* sv = nullptr;
     if (lk >= 0) {
         nl = nr[sep];
-        sv = G.sepv + (size_t)lk * 4 * kLanes;
+        sv = G.sepv + (size_t)lk * (TEAM ? kTeamRows : 4) * kLanes;
     }
     SpineCarry<R> k;
     k.reset();
@@ -726,7 +798,8 @@ __device__ __forceinline__ void channels_item(const SimArgs<R>& A, const Group<R
         if (p < n_light) {
             eliminate_node(G, nd, i, x, rhs, e, k.x, k.r);
         } else if (p < n_sep) {
-            store_row(G, i, x, rhs, e);
+            if constexpr (TEAM) store_row_at(G.sepv + (size_t)(sepk * kTeamRows + 4) * kLanes, x, rhs, e);
+            else store_row(G, i, x, rhs, e);
             e_l = e;
             k.reset();
         } else {
@@ -736,82 +809,143 @@ __device__ __forceinline__ void channels_item(const SimArgs<R>& A, const Group<R
 }
 
 // S2 through shared memory.  Every warp stages a share of the separators
-// at once (their accumulated rows, couplings and voltages: one memory round
-// trip for all of them), then warp 0 runs the skeleton's elimination and
-// back-substitution on the staged rows, where each separator's dependence
-// on its children goes through shared memory instead of a global
-// read-modify-write, and writes back dV and V.
-template <typename R>
+// (their accumulated rows and couplings, and in the first step of a launch
+// their voltages: one memory round trip for all of them).  The skeleton is
+// then eliminated chain by chain (SkelNode), a warp per group of chains and
+// one barrier per chain level, deepest first: along a chain what a node adds
+// to its parent stays in registers and the next node's numbers are read one
+// node ahead, so a step of the chain is an FP64 sum, a reciprocal and a few
+// products; a chain's head adds to its parent's accumulators.  The
+// back-substitution walks the chains down the same way, and at last every
+// warp updates the voltages of a
+// share of the separators.  One warp walking all separators one by one took
+// 19 % of the HH cell's step at one CTA of 15 warps, and would take more than
+// the items themselves when a team of CTAs shares the tree.
+// team: the CTAs of a team each run the whole solve on the same numbers;
+// rd, clr: the junction accumulators this step reads and those it clears
+// (the same ones without a team).
+template <bool TEAM, typename T>
+__device__ __forceinline__ T ld_team(const T* p) {  // a team's numbers come from other SMs: read past the L1
+    if constexpr (TEAM) return __ldcg(p);
+    else return *p;
+}
+template <typename R, bool TEAM>
 __device__ __forceinline__ void skeleton_staged(const SimArgs<R>& A, const Group<R>& G, const NodeRec<R>* nr,
-                                                char* smem, bool rec_now, float* trace, int& bad) {
+                                                const Skel<R>& K, double* rd, double* clr, const R* sepv, bool load_v,
+                                                int rank, bool rec_now, float* trace, int& bad) {
     using M = Math<R>;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int S = A.n_seps;
-    double* acx = (double*)(smem + SmemPlan<R>::nodes(A.n_nodes));
-    double* acr = acx + (size_t)S * kLanes;
-    R* sA = (R*)(acr + (size_t)S * kLanes);
-    R* sB = sA + (size_t)S * kLanes;
-    R* sE = sB + (size_t)S * kLanes;
-    R* sV = sE + (size_t)S * kLanes;
-    R* sC = sV + (size_t)S * kLanes;
-    for (int k = w; k < S; k += nw) {
-        const DevSep sp = A.seps[k];
+#pragma unroll(TEAM ? 4 : 2)
+    for (int q = w; q < S; q += nw) {
+        const SkelNode sp = K.nd[q];
         const NodeRec<R> s = nr[sp.node];
-        const R* row = G.scr + (size_t)sp.node * 3 * kLanes;
-        double* ja = G.jacc + (size_t)(2 * s.jslot) * kLanes;
-        const R* vo = G.vbuf + (size_t)sp.node * 2 * kLanes;
-        double x = (double)row[0] + ja[0], rh = (double)row[kLanes] + ja[kLanes];
-        R a = s.a, b = s.b, e = row[2 * kLanes];
+        const size_t jo = (size_t)(2 * sp.jslot) * kLanes;
+        const R* sv = sepv + (size_t)sp.k * (TEAM ? kTeamRows : 4) * kLanes;
+        const R* row = TEAM ? sv + 4 * kLanes : G.scr + (size_t)sp.node * 3 * kLanes;
+        double x = (double)ld_team<TEAM>(row) + ld_team<TEAM>(rd + jo);
+        double rh = (double)ld_team<TEAM>(row + kLanes) + ld_team<TEAM>(rd + jo + kLanes);
+        R a = s.a, b = s.b, e = ld_team<TEAM>(row + 2 * kLanes);
+        const R la = ld_team<TEAM>(sv), lb = ld_team<TEAM>(sv + kLanes);
+        const R lx = ld_team<TEAM>(sv + 2 * kLanes), lr = ld_team<TEAM>(sv + 3 * kLanes);
         if (sp.seg >= 0) {
-            const R* sv = G.sepv + (size_t)k * 4 * kLanes;
-            a = sv[0];
-            b = sv[kLanes];
-            x += (double)sv[2 * kLanes];
-            rh += (double)sv[3 * kLanes];
+            a = la;
+            b = lb;
+            x += (double)lx;
+            rh += (double)lr;
             e = 0;  // the segment already folded this node's axial term in
         }
-        ja[0] = 0.0;
-        ja[kLanes] = 0.0;
-        const size_t o = (size_t)k * kLanes + lane;
-        acx[o] = x;
-        acr[o] = rh;
-        sA[o] = a;
-        sB[o] = b;
-        sE[o] = e;
-        sV[o] = vo[0];
-        sC[o] = vo[kLanes];
+        if (!TEAM || rank == 0) {
+            clr[jo] = 0.0;
+            clr[jo + kLanes] = 0.0;
+        }
+        const int o = q * kLanes + lane;
+        K.acx[o] = x;
+        K.acr[o] = rh;
+        K.sA[o] = a;
+        K.sB[o] = b;
+        K.sE[o] = e;
+        if (load_v) {
+            const R* vo = G.vbuf + (size_t)sp.node * 2 * kLanes;
+            K.sV[o] = vo[0];
+            K.sC[o] = vo[kLanes];
+        }
     }
     __syncthreads();
-    if (w != 0) return;
-    for (int k = S - 1; k >= 0; --k) {
-        const size_t o = (size_t)k * kLanes + lane;
-        const R x = (R)acx[o], rh = (R)acr[o];
-        if (k == 0) {
-            sB[o] = M::dv(rh, x);
-            break;
+    for (int l = A.n_lev - 1; l >= 0; --l) {
+        for (int g = K.lev[l] + w; g < K.lev[l + 1]; g += nw) {
+            for (int c = K.group[g]; c < K.group[g + 1]; ++c) {
+                int o = K.chain[c] * kLanes + lane;
+                const int head = (K.chain[c + 1] - 1) * kLanes + lane;
+                const int up = l > 0 ? K.par[c] * kLanes + lane : head;
+                double x8 = K.acx[o], r8 = K.acr[o], cx = 0, cr = 0;
+                R a = K.sA[o], b = K.sB[o], e = K.sE[o];
+                const double ux = K.acx[up], ur = K.acr[up];
+                for (;;) {
+                    const int on = o < head ? o + kLanes : o;
+                    const double x8n = K.acx[on], r8n = K.acr[on];
+                    const R an = K.sA[on], bn = K.sB[on], en = K.sE[on];
+                    const R x = (R)(x8 + cx), rh = (R)(r8 + cr);
+                    if (l == 0 && o == head) {  // the root
+                        K.sE[o] = M::dv(rh, x);
+                        break;
+                    }
+                    const R inv = M::rc(x - a);
+                    const R rr = rh * inv;
+                    K.sA[o] = a * inv;
+                    K.sB[o] = rr;
+                    cx = (double)(-b * (x * inv));
+                    cr = (double)(e - b * rr);
+                    if (o == head) {
+                        K.acx[up] = ux + cx;
+                        K.acr[up] = ur + cr;
+                        break;
+                    }
+                    o = on;
+                    x8 = x8n;
+                    r8 = r8n;
+                    a = an;
+                    b = bn;
+                    e = en;
+                }
+            }
         }
-        const R Acp = sA[o], Bcp = sB[o], e_up = sE[o];
-        const R inv = M::rc(x - Acp);
-        const R rr = rh * inv, cc = Acp * inv;
-        sA[o] = cc;
-        sB[o] = rr;
-        const size_t op = (size_t)A.seps[k].par * kLanes + lane;
-        acx[op] += (double)(-Bcp * (x * inv));
-        acr[op] += (double)(e_up - Bcp * rr);
+        __syncthreads();
     }
-    for (int k = 0; k < S; ++k) {
-        const DevSep sp = A.seps[k];
-        const NodeRec<R> s = nr[sp.node];
-        const size_t o = (size_t)k * kLanes + lane;
-        const R x = k == 0 ? sB[o] : sB[o] - sA[o] * sE[(size_t)sp.par * kLanes + lane];
-        sE[o] = x;
-        G.jx[(size_t)s.jslot * kLanes] = x;
-        R* vo = G.vbuf + (size_t)sp.node * 2 * kLanes;
-        R V = sV[o], vc = sC[o];
+    for (int l = 0; l < A.n_lev; ++l) {
+        for (int c = K.group[K.lev[l]] + w; c < K.group[K.lev[l + 1]]; c += nw) {
+            const int q0 = K.chain[c];
+            int q = K.chain[c + 1] - 1;
+            R x = K.sE[(l == 0 ? q : K.par[c]) * kLanes + lane];
+            if (l == 0) --q;
+            if (q < q0) continue;
+            int o = q * kLanes + lane;
+            R r = K.sB[o], cc = K.sA[o];
+            for (; q >= q0; --q, o -= kLanes) {
+                const int on = q > q0 ? o - kLanes : o;
+                const R rn = K.sB[on], cn = K.sA[on];
+                x = r - cc * x;
+                K.sE[o] = x;
+                r = rn;
+                cc = cn;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll 2
+    for (int q = w; q < S; q += nw) {
+        const SkelNode sp = K.nd[q];
+        const int o = q * kLanes + lane;
+        const R x = K.sE[o];
+        G.jx[(size_t)sp.jslot * kLanes] = x;
+        R V = K.sV[o], vc = K.sC[o];
         kahan_add(V, vc, x);
+        K.sV[o] = V;
+        K.sC[o] = vc;
+        R* vo = G.vbuf + (size_t)sp.node * 2 * kLanes;
         vo[0] = V;
         vo[kLanes] = vc;
-        record(A, s, V, rec_now, trace);
+        record(A, nr[sp.node], V, rec_now && rank == 0, trace);
         bad |= v_bad(V);
     }
 }
@@ -819,10 +953,10 @@ __device__ __forceinline__ void skeleton_staged(const SimArgs<R>& A, const Group
 // Work item k of a step: an item's back-substitution pass, then its channel
 // pass; k >= n_comps: a separator linked directly to the skeleton (its
 // channel update and its row for the skeleton solve).
-template <typename R, int MS, typename Classes, bool TI>
+template <typename R, int MS, typename Classes, bool TI, bool TEAM = false>
 __device__ __forceinline__ void run_item(const SimArgs<R>& A, const Group<R>& G, const NodeRec<R>* nr, int k,
                                          R dt, R dtn_inv, R istim_amp, bool rec_now, float* trace, int& bad) {
-    int lo = 0, hi = 0, sep = -1, r = 0, lk = -1;
+    int lo = 0, hi = 0, sep = -1, sepk = k - A.n_comps, r = 0, lk = -1;
     if (k < A.n_comps) {
         const DevComp c = A.comps[k];
         backsub_item<R, TI>(A, G, nr, c, rec_now, trace, bad);
@@ -831,17 +965,18 @@ __device__ __forceinline__ void run_item(const SimArgs<R>& A, const Group<R>& G,
         sep = c.l;
         r = c.r;
         lk = c.lk;
+        sepk = lk;
     } else {
-        const DevSep sp = A.seps[k - A.n_comps];
+        const DevSep sp = A.seps[sepk];
         if (sp.seg < 0) sep = sp.node;  // separators ending a segment are their segment's
     }
-    channels_item<R, MS, Classes, TI>(A, G, nr, lo, hi, sep, r, lk, dt, dtn_inv, istim_amp);
+    channels_item<R, MS, Classes, TI, TEAM>(A, G, nr, lo, hi, sep, sepk, r, lk, dt, dtn_inv, istim_amp);
 }
 
-// Per timestep (two barriers, three with a staged skeleton):
+// Per timestep (two barriers, more with a staged skeleton):
 //   S2  warp 0 solves the skeleton (the separators, a few dozen nodes) with
 //       the reduced couplings of the segments, and updates (and records)
-//       their V; staged (skeleton_staged), all warps first load its rows
+//       their V; staged (skeleton_staged), all warps share it
 //   S3  all warps take items from a queue, largest first: an item's
 //       back-substitution pass, then its channel pass (channel update,
 //       next-step assembly and elimination node by node, above); each
@@ -853,16 +988,53 @@ __device__ __forceinline__ void run_item(const SimArgs<R>& A, const Group<R>& G,
 // operations as one launch.  n_steps timesteps of group g; the items are
 // shared by however many warps the CTA has (the split was sized for
 // A.n_warps).
-template <typename R, int MS, typename Classes>
+//
+// TEAM: a cluster of A.team CTAs on as many SMs shares the group's tree, for
+// batches of too few groups to give every SM one (a group alone is bound by
+// its SM's instruction issue).  The host deals the items to the CTAs; a
+// node's rows are only ever touched by its item's CTA.  What crosses CTAs
+// are the separators' numbers: their FP64 accumulators, segment links and
+// assembled rows, kept in three copies used in turn (step k of a launch
+// reads copy k % 3, adds to copy (k + 1) % 3 and clears copy (k + 2) % 3,
+// which was read a step ago), so that one cluster barrier per step orders
+// everything: no CTA writes what another may still read.  Every CTA solves
+// the whole skeleton itself from the same numbers (bit for bit the same
+// dV), keeps the separators' V in its own shared memory, and writes dV and V
+// of all of them for its own items to read.  A launch starts from and ends
+// on copy 0.
+__device__ __forceinline__ int cluster_rank() {
+    int r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename R, int MS, typename Classes, bool TEAM = false>
 __device__ __forceinline__ void advance_body(const SimArgs<R>& A, int g, int t0, int n_steps, char* smem,
                                              int* ctr) {
-    const Group<R> G = group_of(A, g);
+    Group<R> G = group_of(A, g);
     const int w = threadIdx.x >> 5;
     const NodeRec<R>* nr = stage_nodes(A, smem);
+    const Skel<R> K(A, smem);
+    if (A.s2_stage) K.load_tables(A);
     if (threadIdx.x == 0) { ctr[0] = 0; ctr[1] = 0; }
     __syncthreads();
     int bad = 0;
-    const int n_items = A.n_comps + A.n_seps;
+    int n_items = A.n_comps + A.n_seps, rank = 0;
+    const int* my_items = nullptr;
+    double* jacc0 = G.jacc;  // the accumulators' copies
+    R* sepv0 = G.sepv;
+    const size_t jcopy = (size_t)2 * A.n_jslots * kLanes, scopy = (size_t)kTeamRows * A.n_seps * kLanes;
+    if constexpr (TEAM) {
+        rank = cluster_rank();
+        my_items = A.team_items + A.team + 1 + A.team_items[rank];
+        n_items = A.team_items[rank + 1] - A.team_items[rank];
+        jacc0 = A.jacc + (size_t)g * 3 * jcopy + (threadIdx.x & 31);
+        sepv0 = A.sepv + (size_t)g * 3 * scopy + (threadIdx.x & 31);
+    }
+    int cp = 0;  // TEAM: the copy this step reads
     for (int t = t0; t < t0 + n_steps; ++t) {
         // this step's queue is ctr[t & 1]; the other counter was last used
         // by the previous step's queue, which the barrier ended
@@ -873,8 +1045,15 @@ __device__ __forceinline__ void advance_body(const SimArgs<R>& A, int g, int t0,
         float* trace;
         step_inputs(A, G, t, false, dt, dtn_inv, istim_amp, rec_now, trace);
         // S2: skeleton
-        if (A.s2_stage) {
-            skeleton_staged<R>(A, G, nr, smem, rec_now, trace, bad);
+        if constexpr (TEAM) {
+            const int nx = cp == 2 ? 0 : cp + 1, ol = nx == 2 ? 0 : nx + 1;
+            skeleton_staged<R, true>(A, G, nr, K, jacc0 + cp * jcopy, jacc0 + ol * jcopy, sepv0 + cp * scopy, t == t0,
+                                     rank, rec_now, trace, bad);
+            G.jacc = jacc0 + nx * jcopy;
+            G.sepv = sepv0 + nx * scopy;
+            cp = nx;
+        } else if (A.s2_stage) {
+            skeleton_staged<R, false>(A, G, nr, K, G.jacc, G.jacc, G.sepv, t == t0, 0, rec_now, trace, bad);
         } else if (w == 0) {
             using M = Math<R>;
             for (int k = A.n_seps - 1; k >= 0; --k) {
@@ -927,8 +1106,25 @@ __device__ __forceinline__ void advance_body(const SimArgs<R>& A, int g, int t0,
         __syncthreads();
         // S3: items
         for (int k = next_item(q); k < n_items; k = next_item(q))
-            run_item<R, MS, Classes, false>(A, G, nr, k, dt, dtn_inv, istim_amp, rec_now, trace, bad);
-        __syncthreads();
+            run_item<R, MS, Classes, false, TEAM>(A, G, nr, TEAM ? my_items[k] : k, dt, dtn_inv, istim_amp, rec_now,
+                                                  trace, bad);
+        if constexpr (TEAM) cluster_barrier();
+        else __syncthreads();
+    }
+    if constexpr (TEAM) {
+        if (cp != 0 && rank == 0) {  // back to copy 0, copy 1 cleared for the next launch's first step
+            for (int k = w; k < A.n_seps; k += blockDim.x >> 5) {
+                const size_t jo = (size_t)(2 * nr[A.seps[k].node].jslot) * kLanes;
+                for (int r = 0; r < 2; ++r) {
+                    jacc0[jo + r * kLanes] = __ldcg(jacc0 + cp * jcopy + jo + r * kLanes);
+                    jacc0[jcopy + jo + r * kLanes] = 0.0;
+                }
+                for (int r = 0; r < kTeamRows; ++r) {
+                    const size_t o = (size_t)(k * kTeamRows + r) * kLanes;
+                    sepv0[o] = __ldcg(sepv0 + cp * scopy + o);
+                }
+            }
+        }
     }
     // any warp that saw a non-finite voltage of this group's instance (lane)
     if (bad) A.bad[G.inst] = 1;
