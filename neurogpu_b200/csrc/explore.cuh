@@ -1,4 +1,5 @@
-// Parameter-exploration score of many voltage traces, one thread per trace:
+// Parameter-exploration score of many voltage traces, a warp per 32 traces and
+// stretch of time:
 // the number of peaks of dV/dt that scipy.signal.find_peaks(dvdt, height,
 // distance) returns (scipy 1.x; not vendored in the reference).  This is the
 // score of the reference's exploration run (GUI/plot_param_explor.py:77-107:
@@ -26,12 +27,23 @@
 // matches.
 //
 // Scratch: the candidate peaks' sample positions, [cap][n_traces] int32 with
-// cap = n_samples / 2 + 1 (peaks are at least two samples apart), written and
-// read by the trace's own thread only; threads of a warp touch one row at a
-// time, consecutive traces.
+// cap = n_samples / 2 + 1 (peaks are at least two samples apart); threads of a
+// warp touch one row at a time, consecutive traces.
+//
+// A trace is scanned in stretches side by side (k_dvdt_peaks): whether a rise
+// at sample j starts a peak depends on x[j-1], x[j] and the first later
+// sample that differs from x[j], so the stretch that holds j decides alone.
+// The scan compares differences instead of quotients, which order alike
+// unless two different differences round to one quotient; that takes
+// differences within 2^-51 of each other, which samples with 2^-17 <= |v| <
+// 2^8 cannot have (their differences are exact multiples of 2^-40 below
+// 2^9).  Around any other sample (0, NaN, infinities, beyond 256 mV) the
+// quotients themselves are compared.
 #pragma once
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 namespace ngpu {
 
@@ -54,66 +66,10 @@ __host__ __device__ __forceinline__ double dvdt_at(const PeakArgs& a, const floa
 
 // Removed peaks carry kPeakGone in their position word, kept ones kPeakKept.
 constexpr int32_t kPeakGone = 1 << 30, kPeakKept = 1 << 29;
-// Samples loaded ahead per thread (rows in flight; the scan is latency-bound).
-constexpr int kPeakChunk = 32;
 
-// The score of trace t (one thread's work; host-callable for tests).
-__host__ __device__ inline int dvdt_peaks_trace(const PeakArgs& a, int t) {
-    const float* v = a.v + (int64_t)t * a.stride_trace;
-    int32_t* pos = a.pos + t;
-    const int64_t ps = a.n_traces;
-    const int nx = a.n_samples - 1;  // dvdt samples
-    // 1 + 2: local maxima at or above the height, in position order.  One
-    // pass over the samples, kPeakChunk loads in flight: x[j] is formed from
-    // samples j and j + 1 as they arrive, and a candidate is a rising sample
-    // (x[j-1] < x[j], 1 <= j <= nx - 2) whose run of equal values ends in a
-    // smaller sample (a peak at the run's middle), in a larger one (no peak;
-    // that sample is the next candidate) or in a NaN or the trace's end (no
-    // peak).  These are the decisions of scipy's scan, taken as the samples
-    // stream by instead of by looking ahead.
-    int m = 0;
-    if (nx >= 3) {
-        float vprev = v[0];
-        double xprev = 0.0, pv = 0.0;
-        bool cand = false;
-        int i0 = 0;
-        for (int s0 = 1; s0 < a.n_samples; s0 += kPeakChunk) {
-            float buf[kPeakChunk];
-#pragma unroll
-            for (int u = 0; u < kPeakChunk; ++u)
-                if (s0 + u < a.n_samples) buf[u] = v[(int64_t)(s0 + u) * a.stride_sample];
-#pragma unroll
-            for (int u = 0; u < kPeakChunk; ++u) {
-                const int j = s0 + u - 1;  // dvdt sample of samples j, j + 1
-                if (j + 1 < a.n_samples) {
-                    const double x = ((double)buf[u] - (double)vprev) / a.dt;
-                    vprev = buf[u];
-                    if (j > 0) {
-                        if (cand) {
-                            if (x == pv) {
-                                // the run goes on
-                            } else if (x < pv) {
-                                if (pv >= a.height && m < a.cap) pos[(int64_t)m++ * ps] = (i0 + j - 1) / 2;
-                                cand = false;
-                            } else if (x > pv) {
-                                cand = j <= nx - 2;
-                                i0 = j;
-                                pv = x;
-                            } else {
-                                cand = false;  // NaN
-                            }
-                        } else if (xprev < x && j <= nx - 2) {
-                            cand = true;
-                            i0 = j;
-                            pv = x;
-                        }
-                    }
-                    xprev = x;
-                }
-            }
-        }
-    }
-    // 3: distance, cluster by cluster
+// Step 3, distance, cluster by cluster, over the m candidates of a trace (in
+// position order, ps elements apart): the peaks kept.
+__host__ __device__ inline int peaks_keep(const PeakArgs& a, const float* v, int32_t* pos, int64_t ps, int m) {
     const int d = a.distance;
     int kept = 0;
     int c0 = 0;
@@ -158,9 +114,180 @@ __host__ __device__ inline int dvdt_peaks_trace(const PeakArgs& a, int t) {
     return kept;
 }
 
-__global__ void __launch_bounds__(64) k_dvdt_peaks(const PeakArgs a) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < a.n_traces) a.out[t] = dvdt_peaks_trace(a, t);
+// Samples s0 .. s0 + 7 of a trace; row: samples lie side by side and 16-byte
+// aligned (s0 a multiple of 8), two vector loads.
+constexpr int kTraceBatch = 8;
+__host__ __device__ __forceinline__ void load_batch(const float* v, int64_t st, bool row, int s0,
+                                                    float (&x)[kTraceBatch]) {
+#ifdef __CUDA_ARCH__
+    if (row) {
+        const float4 p = *reinterpret_cast<const float4*>(v + s0), q = *reinterpret_cast<const float4*>(v + s0 + 4);
+        x[0] = p.x, x[1] = p.y, x[2] = p.z, x[3] = p.w, x[4] = q.x, x[5] = q.y, x[6] = q.z, x[7] = q.w;
+        return;
+    }
+#endif
+#pragma unroll
+    for (int u = 0; u < kTraceBatch; ++u) x[u] = v[(int64_t)(s0 + u) * st];
+}
+
+// Samples whose differences order as their quotients do: 2^-17 <= |v| < 2^8.
+// Collected from the bit patterns without the sign: the smallest and the
+// largest (infinities and NaN above every number).
+struct PlainRange {
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
+    __host__ __device__ __forceinline__ void add(float v) {
+        uint32_t b;
+        memcpy(&b, &v, 4);
+        b <<= 1;
+        lo = b < lo ? b : lo;
+        hi = b > hi ? b : hi;
+    }
+    __host__ __device__ __forceinline__ bool ok() const { return lo >= (110u << 24) && hi < (135u << 24); }
+};
+
+// Steps 1 and 2 for the rises of trace t in [lo, hi) (lo a multiple of 8):
+// their peaks' positions go to rows lo / 2, lo / 2 + 1, ... of the scratch
+// (rises are two samples apart, so stretches do not meet); their number.
+// h_lo: differences below it are below the height whatever the rounding.
+// quotients: compare quotients throughout.
+//
+// Between two changes of x all its values are equal, so a rise that the next
+// change undoes is a peak: `up` says that the last change was a rise, at i0.
+// A NaN undoes nothing and ends the run.
+__host__ __device__ inline int peaks_scan(const PeakArgs& a, int t, int lo, int hi, double h_lo, bool quotients,
+                                          bool row) {
+    const float* v = a.v + (int64_t)t * a.stride_trace;
+    const int64_t st = a.stride_sample, ps = a.n_traces;
+    int32_t* pos = a.pos + (int64_t)(lo / 2) * ps + t;
+    const int nx = a.n_samples - 1;
+    const int j0 = lo > 1 ? lo : 1, j1 = hi < nx - 1 ? hi : nx - 1;  // rises in [j0, j1)
+    int m = 0, i0 = 0;
+    if (j0 >= j1) return 0;
+    bool up = false;
+    double vp = (double)v[(int64_t)j0 * st], dp = vp - (double)v[(int64_t)(j0 - 1) * st];
+    // sample j + 1 closes difference j
+    auto peak = [&](int j) {
+        if (dp / a.dt >= a.height) pos[(int64_t)m++ * ps] = (i0 + j - 1) / 2;
+    };
+    auto step = [&](float x, int j) {
+        const double vn = (double)x, d = vn - vp;
+        vp = vn;
+        const bool lt = dp < d, gt = d < dp;
+        if (up & gt & (dp >= h_lo)) peak(j);  // one predicate: a warp rarely goes in
+        up = lt | (up & !gt);
+        i0 = lt ? j : i0;
+        dp = d;
+    };
+    auto step_quotient = [&](float x, int j, bool may_rise) {
+        const double vn = (double)x, d = vn - vp, q = d / a.dt, qp = dp / a.dt;
+        vp = vn;
+        const bool lt = qp < q;
+        if (up && q < qp) peak(j);
+        up = lt ? may_rise : (up && q == qp);
+        if (lt) i0 = j;
+        dp = d;
+    };
+    // samples j0 + 1 .. j1, in whole batches of 8 where they fit
+    int s = j0 + 1;
+    for (; s <= j1 && (s & (kTraceBatch - 1)); ++s) step_quotient(v[(int64_t)s * st], s - 1, true);
+    if (s + kTraceBatch - 1 <= j1) {
+        PlainRange edge;  // the two samples before the first batch
+        edge.add(v[(int64_t)(s - 1) * st]);
+        edge.add(v[(int64_t)(s - 2) * st]);
+        bool plain_before = edge.ok() && !quotients;
+        float nx8[kTraceBatch];
+        load_batch(v, st, row, s, nx8);
+        for (; s + kTraceBatch - 1 <= j1; s += kTraceBatch) {
+            float x[kTraceBatch];
+            PlainRange range;
+#pragma unroll
+            for (int u = 0; u < kTraceBatch; ++u) {
+                x[u] = nx8[u];
+                range.add(x[u]);
+            }
+            if (s + 2 * kTraceBatch - 1 <= j1) load_batch(v, st, row, s + kTraceBatch, nx8);
+            const bool plain = range.ok() && !quotients;
+            if (plain && plain_before) {
+#pragma unroll
+                for (int u = 0; u < kTraceBatch; ++u) step(x[u], s + u - 1);
+            } else {
+                for (int u = 0; u < kTraceBatch; ++u) step_quotient(v[(int64_t)(s + u) * st], s + u - 1, true);
+            }
+            plain_before = plain;
+        }
+    }
+    for (; s <= j1; ++s) step_quotient(v[(int64_t)s * st], s - 1, true);
+    for (; up && s <= nx; ++s) step_quotient(v[(int64_t)s * st], s - 1, false);  // only an open run goes on
+    return m;
+}
+
+// Heights below this difference fail whatever the rounding of the quotient.
+__host__ __device__ inline double peak_h_lo(const PeakArgs& a) {
+    const double hd = a.height * a.dt;
+    return hd - fabs(hd) * 1e-9;
+}
+// Quotients that overflow or vanish (steps no trace has) compare as quotients throughout.
+__host__ __device__ inline bool peak_odd_step(const PeakArgs& a) { return !(a.dt > 1e-100 && a.dt < 1e100); }
+
+// The score of trace t in one stretch (host-callable; the tests' host build).
+__host__ __device__ inline int dvdt_peaks_trace(const PeakArgs& a, int t) {
+    const int m = peaks_scan(a, t, 0, a.n_samples, peak_h_lo(a), peak_odd_step(a), false);
+    return peaks_keep(a, a.v + (int64_t)t * a.stride_trace, a.pos + t, a.n_traces, m);
+}
+
+// Blocks of 32 traces (lane = trace) and blockDim.y stretches of `stretch`
+// samples (even).  What bounds it: reading the traces once.  10,000 traces
+// of 3,168 samples (127 MB): 124 us with cold caches, 52 warp instructions
+// per 32 samples at 43 % issue activity.  One thread per trace (the form
+// this replaces) took 0.79 ms: two warps per SM, each walking 3,168 FP64
+// quotients one after another.
+constexpr int kPeakList = 256;
+__global__ void __launch_bounds__(1024) k_dvdt_peaks(const PeakArgs a, int stretch, int row) {
+    __shared__ int cnt[32][33];
+    extern __shared__ int32_t peak_list[];  // [blockDim.y][kPeakList]
+    const int lane = threadIdx.x, w = threadIdx.y, nw = blockDim.y, t = blockIdx.x * 32 + lane;
+    if (t < a.n_traces)
+        cnt[w][lane] = peaks_scan(a, t, w * stretch, (w + 1) * stretch, peak_h_lo(a), peak_odd_step(a), row);
+    __syncthreads();
+    // the distance rule, a warp per trace: its peaks in order into shared
+    // memory; where no two are close that is their count
+    int32_t* const list = peak_list + w * kPeakList;
+    for (int i = w; i < 32; i += nw) {
+        const int tr = blockIdx.x * 32 + i;
+        if (tr >= a.n_traces) break;
+        int mine = lane < nw ? cnt[lane][i] : 0, upto = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+            if (lane >= o) upto += x;
+        }
+        const int m = __shfl_sync(0xFFFFFFFFu, upto, 31);
+        int32_t* pos = a.pos + tr;
+        const int64_t ps = a.n_traces;
+        const float* v = a.v + (int64_t)tr * a.stride_trace;
+        if (m > kPeakList) {  // too many for the list: closed up in the scratch
+            if (lane == 0) {
+                int n = cnt[0][i];
+                for (int c = 1; c < nw; ++c)
+                    for (int k = 0; k < cnt[c][i]; ++k)
+                        pos[(int64_t)n++ * ps] = pos[(int64_t)(c * (stretch / 2) + k) * ps];
+                a.out[tr] = peaks_keep(a, v, pos, ps, n);
+            }
+            continue;
+        }
+        for (int c = 0; c < nw; ++c) {
+            const int n = cnt[c][i], first = __shfl_sync(0xFFFFFFFFu, upto - mine, c);
+            for (int k = lane; k < n; k += 32) list[first + k] = pos[(int64_t)(c * (stretch / 2) + k) * ps];
+        }
+        __syncwarp();
+        bool close = false;
+        for (int k = lane; k + 1 < m; k += 32) close = close || list[k + 1] - list[k] < a.distance;
+        if (!__any_sync(0xFFFFFFFFu, close)) {
+            if (lane == 0) a.out[tr] = m;
+        } else if (lane == 0) {
+            a.out[tr] = peaks_keep(a, v, list, 1, m);
+        }
+        __syncwarp();
+    }
 }
 
 }  // namespace ngpu

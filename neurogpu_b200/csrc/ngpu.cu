@@ -2058,9 +2058,29 @@ static int feature_args(int32_t n_samples, double dt, double stim_on, double sti
     return NGPU_OK;
 }
 
+// Stretches of time a block's 32 traces are cut into (a warp each): enough
+// for about 16 warps per SM, at least 32 samples each.
+static int trace_stretches(int n_traces, int n_samples) {
+    const int blocks = (n_traces + 31) / 32;
+    int w = 8;
+    while (w < 32 && blocks * w < 16 * kSmCount) w *= 2;
+    while (w > 1 && n_samples < 32 * w) w /= 2;
+    return w;
+}
+
+// Their length, whole batches of 8 samples.
+static int trace_stretch(int n_samples, int w) { return ((n_samples + w - 1) / w + kTraceBatch - 1) / kTraceBatch * kTraceBatch; }
+// Whether a trace's samples lie side by side, every batch on 16 bytes.
+static int trace_rows(const float* v, int64_t stride_trace, int64_t stride_sample) {
+    return stride_sample == 1 && stride_trace % 4 == 0 && (uintptr_t)v % 16 == 0;
+}
+
 static int launch_features(FeatureArgs a, cudaStream_t st) {
     if (a.n_traces < 1) return NGPU_OK;
-    k_trace_features<<<(a.n_traces + 127) / 128, 128, 0, st>>>(a);
+    const int w = trace_stretches(a.n_traces, a.n_samples);
+    const int smem = kFeatBytes * 32 * w;
+    NGPU_CUDA(cudaFuncSetAttribute(k_trace_features, cudaFuncAttributeMaxDynamicSharedMemorySize, kFeatBytes * 32 * w));
+    k_trace_features<<<(a.n_traces + 31) / 32, dim3(32, w), smem, st>>>(a, trace_stretch(a.n_samples, w), trace_rows(a.v, a.stride_trace, a.stride_sample));
     g_launches++;
     NGPU_CUDA(cudaGetLastError());
     return NGPU_OK;
@@ -2120,8 +2140,9 @@ static int launch_dvdt_peaks(PeakArgs a, int64_t scratch_bytes, cudaStream_t st)
         return fail(NGPU_E_INVALID, "dvdt peaks: scratch holds " + std::to_string(scratch_bytes) + " bytes, needs " +
                                         std::to_string(need));
     if (!a.v || !a.out || !a.pos) return fail(NGPU_E_INVALID, "dvdt peaks: null pointer");
-    // 64 threads a CTA: the traces of an exploration (10,000) spread over every SM
-    k_dvdt_peaks<<<(a.n_traces + 63) / 64, 64, 0, st>>>(a);
+    const int w = trace_stretches(a.n_traces, a.n_samples);
+    k_dvdt_peaks<<<(a.n_traces + 31) / 32, dim3(32, w), sizeof(int32_t) * kPeakList * w, st>>>(
+        a, trace_stretch(a.n_samples, w), trace_rows(a.v, a.stride_trace, a.stride_sample));
     g_launches++;
     NGPU_CUDA(cudaGetLastError());
     return NGPU_OK;
