@@ -2823,7 +2823,9 @@ int ngpu_ga_offspring(const double* pop_dev, const int32_t* rank_dev, const doub
     if (n_kids == 0) return NGPU_OK;
     GaVariation a{pop_dev, rank_dev, crowd_dev, mu, n_genes, n_kids, low, up, eta_c, eta_m, cx_prob, p_mut,
                   ga_key(seed, generation), kids_dev};
-    k_ga_offspring<<<(n_kids + 127) / 128, 128, 0, (cudaStream_t)cuda_stream>>>(a);
+    const int64_t threads = (int64_t)n_kids * n_genes;
+    if (threads > (int64_t)0x7FFFFFFF * 128) return fail(NGPU_E_INVALID, "ga_offspring: too many children");
+    k_ga_offspring<<<(unsigned)((threads + 127) / 128), 128, 0, (cudaStream_t)cuda_stream>>>(a);
     g_launches++;
     NGPU_CUDA(cudaGetLastError());
     return NGPU_OK;
@@ -2836,6 +2838,18 @@ int ngpu_ga_select_truncation(const double* score_dev, int32_t n, int32_t mu, in
     cudaStream_t st = (cudaStream_t)cuda_stream;
     int rc = NGPU_OK;
     StreamScratch ws(st);
+    if (n <= kGaSmallMax) {  // places by counting; n^2 comparisons, a sort's launches above
+        uint64_t* key = ws.get<uint64_t>(n, &rc);
+        int32_t* seat = ws.get<int32_t>(n, &rc);
+        if (rc != NGPU_OK) return rc;
+        const int b = (n + 255) / 256;
+        k_ga_score_keys<<<b, 256, 0, st>>>(score_dev, n, key, seat);
+        k_ga_seats_key<<<dim3(b, (n + kGaCount - 1) / kGaCount), 256, 0, st>>>(key, nullptr, n, seat);
+        k_ga_take_seats<<<b, 256, 0, st>>>(seat, n, mu, out_idx_dev);
+        g_launches += 3;
+        NGPU_CUDA(cudaGetLastError());
+        return NGPU_OK;
+    }
     const uint32_t n2 = pow2_at_least(n);
     GaSortSlice s{ws.get<uint64_t>(n2, &rc), ws.get<uint64_t>(n2, &rc), ws.get<uint32_t>(n2, &rc)};
     if (rc != NGPU_OK) return rc;
@@ -2843,6 +2857,73 @@ int ngpu_ga_select_truncation(const double* score_dev, int32_t n, int32_t mu, in
     g_launches += ga_sort(s, n2, 1, st);
     k_ga_take<<<grid_for(mu, 256), 256, 0, st>>>(s.idx, mu, out_idx_dev);
     g_launches += 2;
+    NGPU_CUDA(cudaGetLastError());
+    return NGPU_OK;
+}
+
+extern "C++" {
+// k_ga_dominance_ranks for the smallest word count that holds q
+template <int Q>
+static void launch_dominance_ranks(const uint32_t* sorted2, const uint32_t* sum, int n, int q, uint32_t* dom,
+                                   cudaStream_t st) {
+    if constexpr (Q < 96) {
+        if (q > Q) return launch_dominance_ranks<(Q < 64 ? 2 * Q : 96)>(sorted2, sum, n, q, dom, st);
+    }
+    k_ga_dominance_ranks<Q><<<dim3((n + 255) / 256, (n + ga_dom_j(Q) - 1) / ga_dom_j(Q)), 256, 0, st>>>(sorted2, sum, n, q, dom);
+}
+}
+
+// NSGA-II selection of n <= kGaSmallMax individuals.
+static int select_nsga2_small(const double* obj, int n, int m, int mu, int32_t* out_idx, int32_t* rank, double* crowd,
+                              int32_t* n_fronts, cudaStream_t st) {
+    int rc = NGPU_OK;
+    StreamScratch ws(st);
+    const int W = (n + 31) / 32, q = (m + 1) / 2, b = (n + 255) / 256;
+    const uint32_t tile = std::min<uint32_t>(kGaTile, std::max<uint32_t>(64, pow2_at_least(n)));
+    const int tiles = (int)((n + tile - 1) / tile);
+    const dim3 pairs(b, (n + kGaCount - 1) / kGaCount);
+    uint16_t* order = ws.get<uint16_t>((size_t)m * n, &rc);
+    uint16_t* in_fronts = ws.get<uint16_t>((size_t)m * n, &rc);
+    uint64_t* tile_key = ws.get<uint64_t>((size_t)m * tiles * tile, &rc);
+    uint16_t* tile_idx = ws.get<uint16_t>((size_t)m * tiles * tile, &rc);
+    uint32_t* rank2 = ws.get<uint32_t>((size_t)q * n, &rc);
+    uint32_t* sorted2 = ws.get<uint32_t>((size_t)q * n, &rc);
+    uint32_t* sum = ws.get<uint32_t>(n, &rc);
+    uint32_t* sorted_sum = ws.get<uint32_t>(n, &rc);
+    int32_t* seat = ws.get<int32_t>(n, &rc);
+    int32_t* who = ws.get<int32_t>(n, &rc);
+    uint32_t* dom = ws.get<uint32_t>((size_t)n * W, &rc);
+    uint32_t* mask = ws.get<uint32_t>((size_t)3 * W, &rc);
+    int32_t* start = ws.get<int32_t>((size_t)n + 1, &rc);
+    double* contrib = ws.get<double>((size_t)m * n, &rc);
+    uint64_t* key = ws.get<uint64_t>(n, &rc);
+    if (rc != NGPU_OK) return rc;
+    const GaOrderArgs oa{obj, rank, n_fronts, n, m, tile, tile_key, tile_idx, order, (uint16_t*)rank2, in_fronts};
+    k_ga_tiles<false><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
+    k_ga_places<false><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
+    k_ga_rank_sums<<<b, 256, 0, st>>>(rank2, n, q, sum, seat);
+    k_ga_seats_sum<<<pairs, 256, 0, st>>>(sum, n, seat);
+    k_ga_seat_ranks<<<b, 256, 0, st>>>(rank2, sum, seat, n, q, sorted2, sorted_sum, who);
+    launch_dominance_ranks<1>(sorted2, sorted_sum, n, q, dom, st);
+    {
+        // cooperative: every CTA resident at once (the grid barrier needs it)
+        int dev = 0, sms = 0, per_sm = 0;
+        NGPU_CUDA(cudaGetDevice(&dev));
+        NGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        NGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ga_fronts_count, kGaDomThreads, 0));
+        const int blocks = (4 * n + kGaDomThreads - 1) / kGaDomThreads;
+        if (sms * per_sm < blocks) return fail(NGPU_E_CUDA, "ga_select_nsga2: the front kernel cannot be resident");
+        GaFrontCountArgs fa{dom, who, n, W, rank, mask, start, n_fronts};
+        void* args[] = {&fa};
+        NGPU_CUDA(cudaLaunchCooperativeKernel((const void*)k_ga_fronts_count, dim3(blocks), dim3(kGaDomThreads), args, 0, st));
+    }
+    k_ga_tiles<true><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
+    k_ga_places<true><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
+    k_ga_crowd_small<<<dim3(b, m), 256, 0, st>>>(GaCrowdSmallArgs{obj, in_fronts, rank, start, n, m, contrib});
+    k_ga_crowd_seats<<<b, 256, 0, st>>>(contrib, rank, start, n, m, crowd, key, seat);
+    k_ga_seats_key<<<pairs, 256, 0, st>>>(key, rank, n, seat);
+    k_ga_take_seats<<<b, 256, 0, st>>>(seat, n, mu, out_idx);
+    g_launches += 13;
     NGPU_CUDA(cudaGetLastError());
     return NGPU_OK;
 }
@@ -2855,6 +2936,8 @@ int ngpu_ga_select_nsga2(const double* obj_dev, int32_t n, int32_t m, int32_t mu
         return fail(NGPU_E_INVALID, "ga_select_nsga2: 1 <= mu <= n <= " + std::to_string(32 * kGaMaxWords));
     if (m < 1 || m > 192) return fail(NGPU_E_INVALID, "ga_select_nsga2: 1..192 objectives");
     cudaStream_t st = (cudaStream_t)cuda_stream;
+    if (n <= kGaSmallMax)
+        return select_nsga2_small(obj_dev, n, m, mu, out_idx_dev, rank_dev, crowd_dev, n_fronts_dev, st);
     int rc = NGPU_OK;
     StreamScratch ws(st);
     const int W = (n + 31) / 32;
