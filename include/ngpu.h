@@ -387,6 +387,39 @@ int ngpu_gemm_bf16_tn(const void *A, const void *B, int32_t M, int32_t N, int32_
 int ngpu_gemm_error(int32_t *flag);
 
 /*
+ * The surrogate network (in -> width -> width -> width -> out, GELU) on the
+ * GEMMs above, a whole prediction, gradient or optimizer step per call; all
+ * pointers device memory, the pointer arrays host memory.  wb[l]: bf16
+ * weights [rows][cols] (l = 0: [width][k_in], 1, 2: [width][width], 3:
+ * [n_out_p][width]); wtb[l]: their transposes (3: [width][64], zero-padded);
+ * b[l]: biases.  k_in, width: multiples of 64, n_out_p of 32 (at most 64 for
+ * gradients).  X [M][n_in],
+ * Y [M][n_out]; x_mu, x_sd, y_mu, y_sd: standardisation, or NULL.
+ *   ngpu_mlp_predict  out [M][n_out]
+ *   ngpu_mlp_grads    mean squared error on standardised targets (weight [M]
+ *                     or NULL multiplies the differences), gradients gw[l],
+ *                     gb[l] in the weights' shapes
+ *   ngpu_mlp_adam     p, g, m, v: 4 weights, then 4 biases; c1 = 1 - b1^t, c2
+ *                     = 1 - b2^t; wb, wtb receive the new weights' copies;
+ *                     what lies past n_in inputs and n_out outputs becomes 0
+ *   workspace: ngpu_mlp_workspace_bytes, 256-byte aligned, used on the stream
+ * No counterpart in the reference.
+ */
+int64_t ngpu_mlp_workspace_bytes(int32_t M, int32_t width, int32_t k_in, int32_t n_out_p, int32_t train);
+int ngpu_mlp_predict(const float *X, int32_t M, int32_t n_in, const float *x_mu, const float *x_sd,
+                     const void *const *wb, const float *const *b, int32_t width, int32_t k_in, int32_t n_out,
+                     int32_t n_out_p, const float *y_mu, const float *y_sd, void *ws, int64_t ws_bytes, float *out,
+                     void *cuda_stream);
+int ngpu_mlp_grads(const float *X, const float *Y, const float *weight, int32_t M, int32_t n_in, const float *x_mu,
+                   const float *x_sd, const float *y_mu, const float *y_sd, const void *const *wb,
+                   const void *const *wtb, const float *const *b, int32_t width, int32_t k_in, int32_t n_out,
+                   int32_t n_out_p, void *ws, int64_t ws_bytes, float *loss, float *const *gw, float *const *gb,
+                   void *cuda_stream);
+int ngpu_mlp_adam(float *const *p, const float *const *g, float *const *m, float *const *v, void *const *wb,
+                  void *const *wtb, int32_t n_in, int32_t width, int32_t k_in, int32_t n_out, int32_t n_out_p, float lr,
+                  float b1, float b2, float eps, float c1, float c2, void *cuda_stream);
+
+/*
  * Genetic-algorithm steps on the device (all pointers device memory, all
  * objectives minimised), so that a generation needs no host round trip.
  * They replace the host-side DEAP operators between simulator calls

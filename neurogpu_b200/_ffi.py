@@ -67,6 +67,11 @@ def lib() -> C.CDLL:
             "ngpu_batch_run_graph": (C.c_int, [P, F32, I32, I32, P]),
             "ngpu_gemm_bf16_tn": (C.c_int, [P, P, I32, I32, I32, I32, I32, I32, I32, P, P, P, I32, I32, P, P, P]),
             "ngpu_gemm_error": (C.c_int, [P]),
+            "ngpu_mlp_workspace_bytes": (I64, [I32, I32, I32, I32, I32]),
+            "ngpu_mlp_predict": (C.c_int, [P, I32, I32, P, P, P, P, I32, I32, I32, I32, P, P, P, I64, P, P]),
+            "ngpu_mlp_grads": (C.c_int, [P, P, P, I32, I32, P, P, P, P, P, P, P, I32, I32, I32, I32, P, I64, P, P, P,
+                                         P]),
+            "ngpu_mlp_adam": (C.c_int, [P, P, P, P, P, P, I32, I32, I32, I32, I32, F32, F32, F32, F32, F32, F32, P]),
             "ngpu_sim_destroy": (C.c_int, [P]),
             "ngpu_sim_set_params": (C.c_int, [P, P, I32]),
             "ngpu_sim_set_stimulus": (C.c_int, [P, I32, P, P, I32, F32, I32]),

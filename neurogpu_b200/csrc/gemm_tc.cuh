@@ -54,6 +54,7 @@ enum GemmEpilogue : int {
     kEpiBias = 2,       // out_f32[m][n] = D + bias[n]
     kEpiGeluGrad = 3,   // dz = D * gelu'(zin[m][n]): out_bf16 = dz, out_bf16_t[n][m] = dz
     kEpiSplitAdd = 4,   // out_f32[m][n] += D over this CTA's slice of K (split-K; out_f32 zeroed first)
+    kEpiGelu = 5,       // out_bf16[m][n] = gelu(D + bias[n]) alone: a prediction needs neither z nor the transpose
 };
 
 struct GemmArgs {
@@ -174,6 +175,8 @@ __device__ __forceinline__ void epi_one(const GemmArgs& g, float* sp, size_t o, 
         g.out_f32[o] = d + g.bias[n];
     } else if constexpr (EPI == kEpiSplitAdd) {
         atomicAdd(g.out_f32 + o, d);
+    } else if constexpr (EPI == kEpiGelu) {
+        g.out_bf16[o] = __float2bfloat16_rn(gelu_tanh(d + g.bias[n]));
     } else if constexpr (EPI == kEpiBiasGelu) {
         const float z = d + g.bias[n];
         const __nv_bfloat16 h = __float2bfloat16_rn(gelu_tanh(z));
@@ -201,10 +204,11 @@ __device__ __forceinline__ void epi_vec4(const GemmArgs& g, float* sp, size_t o,
         *reinterpret_cast<float4*>(g.out_f32 + o) = make_float4(d[0], d[1], d[2], d[3]);
     } else {
         float v[4];
-        if constexpr (EPI == kEpiBiasGelu) {
+        if constexpr (EPI == kEpiBiasGelu || EPI == kEpiGelu) {
             const float4 b = *reinterpret_cast<const float4*>(g.bias + n);
             const float z[4] = {d[0] + b.x, d[1] + b.y, d[2] + b.z, d[3] + b.w};
-            *reinterpret_cast<float4*>(g.out_f32 + o) = make_float4(z[0], z[1], z[2], z[3]);
+            if constexpr (EPI == kEpiBiasGelu)
+                *reinterpret_cast<float4*>(g.out_f32 + o) = make_float4(z[0], z[1], z[2], z[3]);
 #pragma unroll
             for (int q = 0; q < 4; ++q) v[q] = gelu_tanh(z[q]);
         } else {  // kEpiGeluGrad
@@ -217,7 +221,8 @@ __device__ __forceinline__ void epi_vec4(const GemmArgs& g, float* sp, size_t o,
         pk.x = *reinterpret_cast<const uint32_t*>(&lo);
         pk.y = *reinterpret_cast<const uint32_t*>(&hi);
         *reinterpret_cast<uint2*>(g.out_bf16 + o) = pk;
-        sp[0] = __low2float(lo), sp[1] = __high2float(lo), sp[2] = __low2float(hi), sp[3] = __high2float(hi);
+        if constexpr (EPI != kEpiGelu)
+            sp[0] = __low2float(lo), sp[1] = __high2float(lo), sp[2] = __low2float(hi), sp[3] = __high2float(hi);
     }
 }
 

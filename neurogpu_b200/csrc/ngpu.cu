@@ -28,6 +28,7 @@
 #include "features.cuh"
 #include "ga.cuh"
 #include "gemm_tc.cuh"
+#include "mlp.cuh"
 #include "ngpu_jit.h"
 #include "sim_kernels.cuh"
 
@@ -2714,10 +2715,10 @@ static cudaError_t launch_gemm_epi(GemmArgs g, int bn, cudaStream_t st) {
     }
 }
 
-extern "C" int ngpu_gemm_bf16_tn(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t lda,
-                                 int32_t ldb, int32_t epilogue, int32_t bn, float* out_f32, void* out_bf16,
-                                 void* out_bf16_t, int32_t ldo, int32_t ldt, const float* bias, const float* zin,
-                                 void* cuda_stream) {
+// Checks and launch of one GEMM; epilogues up to `last` are known.
+static int gemm_checked(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t lda,
+                        int32_t ldb, int32_t epilogue, int32_t bn, float* out_f32, void* out_bf16, void* out_bf16_t,
+                        int32_t ldo, int32_t ldt, const float* bias, const float* zin, void* cuda_stream, int last) {
     if (!A || !B) return fail(NGPU_E_INVALID, "gemm: null operand");
     if (M < 1 || N < 1 || K < kGemmBK || K % kGemmBK)
         return fail(NGPU_E_INVALID, "gemm: need M, N >= 1 and K a positive multiple of 64");
@@ -2727,11 +2728,13 @@ extern "C" int ngpu_gemm_bf16_tn(const void* A, const void* B, int32_t M, int32_
     if (bn != 32 && bn != 64 && bn != 128 && bn != 256) return fail(NGPU_E_INVALID, "gemm: bn must be 32, 64, 128 or 256");
     const bool need_f32 = epilogue == kEpiStore || epilogue == kEpiBias || epilogue == kEpiBiasGelu ||
                           epilogue == kEpiSplitAdd;
-    const bool need_bf16 = epilogue == kEpiBiasGelu || epilogue == kEpiGeluGrad;
-    if ((need_f32 && !out_f32) || (need_bf16 && (!out_bf16 || !out_bf16_t)) ||
-        ((epilogue == kEpiBias || epilogue == kEpiBiasGelu) && !bias) || (epilogue == kEpiGeluGrad && !zin))
+    const bool need_bf16_t = epilogue == kEpiBiasGelu || epilogue == kEpiGeluGrad;
+    const bool need_bf16 = need_bf16_t || epilogue == kEpiGelu;
+    if (epilogue > last) return fail(NGPU_E_INVALID, "gemm: unknown epilogue");
+    if ((need_f32 && !out_f32) || (need_bf16 && !out_bf16) || (need_bf16_t && !out_bf16_t) ||
+        ((epilogue == kEpiBias || epilogue == kEpiBiasGelu || epilogue == kEpiGelu) && !bias) || (epilogue == kEpiGeluGrad && !zin))
         return fail(NGPU_E_INVALID, "gemm: missing output / bias / pre-activation for the epilogue");
-    if (ldo < N || (need_bf16 && ldt < M)) return fail(NGPU_E_INVALID, "gemm: output leading dimension too small");
+    if (ldo < N || (need_bf16_t && ldt < M)) return fail(NGPU_E_INVALID, "gemm: output leading dimension too small");
     int* err = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void**)&err, g_gemm_err);
     if (e != cudaSuccess) return fail(NGPU_E_CUDA, std::string("gemm: ") + cudaGetErrorString(e));
@@ -2744,9 +2747,194 @@ extern "C" int ngpu_gemm_bf16_tn(const void* A, const void* B, int32_t M, int32_
         case kEpiBias: e = launch_gemm_epi<kEpiBias>(g, bn, st); break;
         case kEpiGeluGrad: e = launch_gemm_epi<kEpiGeluGrad>(g, bn, st); break;
         case kEpiSplitAdd: e = launch_gemm_epi<kEpiSplitAdd>(g, bn, st); break;
+        case kEpiGelu: e = launch_gemm_epi<kEpiGelu>(g, bn, st); break;
         default: return fail(NGPU_E_INVALID, "gemm: unknown epilogue");
     }
     if (e != cudaSuccess) return fail(NGPU_E_CUDA, std::string("gemm launch: ") + cudaGetErrorString(e));
+    return NGPU_OK;
+}
+
+extern "C" int ngpu_gemm_bf16_tn(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t lda,
+                                 int32_t ldb, int32_t epilogue, int32_t bn, float* out_f32, void* out_bf16,
+                                 void* out_bf16_t, int32_t ldo, int32_t ldt, const float* bias, const float* zin,
+                                 void* cuda_stream) {
+    return gemm_checked(A, B, M, N, K, lda, ldb, epilogue, bn, out_f32, out_bf16, out_bf16_t, ldo, ldt, bias, zin,
+                        cuda_stream, kEpiSplitAdd);
+}
+
+// ------------------------------------------------------------------ surrogate network
+namespace {
+
+// Slices of the caller's workspace, 256 bytes apart; with no base, their sum.
+struct Arena {
+    char* base;
+    int64_t used = 0;
+    template <typename T>
+    T* get(size_t count) {
+        const int64_t at = used;
+        used += ((int64_t)(count * sizeof(T)) + 255) / 256 * 256;
+        return base ? (T*)(base + at) : nullptr;
+    }
+};
+
+int64_t pad_to(int64_t n, int64_t m) { return (n + m - 1) / m * m; }
+
+struct MlpPredictWs {
+    __nv_bfloat16 *xb, *h0, *h1;
+    float* y;
+    MlpPredictWs(Arena& a, int64_t Mp, int width, int k_in, int n_out_p)
+        : xb(a.get<__nv_bfloat16>(Mp * k_in)), h0(a.get<__nv_bfloat16>(Mp * width)),
+          h1(a.get<__nv_bfloat16>(Mp * width)), y(a.get<float>(Mp * n_out_p)) {}
+};
+
+struct MlpTrainWs {
+    __nv_bfloat16 *xb, *h[3], *ht[4], *dyb, *dybt, *dzb[3], *dzbt[3];
+    float *z[3], *y, *g4t, *part;
+    unsigned* done;
+    MlpTrainWs(Arena& a, int64_t Mp, int width, int k_in, int n_out_p) {
+        xb = a.get<__nv_bfloat16>(Mp * k_in);
+        ht[0] = a.get<__nv_bfloat16>(Mp * k_in);
+        for (int k = 0; k < 3; ++k) {
+            z[k] = a.get<float>(Mp * width);
+            h[k] = a.get<__nv_bfloat16>(Mp * width);
+            ht[k + 1] = a.get<__nv_bfloat16>(Mp * width);
+            dzb[k] = a.get<__nv_bfloat16>(Mp * width);
+            dzbt[k] = a.get<__nv_bfloat16>(Mp * width);
+        }
+        y = a.get<float>(Mp * n_out_p);
+        dyb = a.get<__nv_bfloat16>(Mp * 64);
+        dybt = a.get<__nv_bfloat16>(Mp * n_out_p);
+        g4t = a.get<float>((size_t)width * n_out_p);
+        part = a.get<float>((size_t)((Mp + kMlpLossRows - 1) / kMlpLossRows) * (1 + n_out_p));
+        done = a.get<unsigned>(1);
+    }
+};
+
+int mlp_check(int64_t M, int n_in, int width, int k_in, int n_out, int n_out_p) {
+    if (M < 1 || M > (1 << 30)) return fail(NGPU_E_INVALID, "mlp: 1 <= rows <= 2^30");
+    if (n_in < 1 || k_in < n_in || k_in % 64 || width < 64 || width % 64 || n_out < 1 || n_out_p < n_out ||
+        n_out_p % 32)
+        return fail(NGPU_E_INVALID, "mlp: k_in and width multiples of 64, n_out_p of 32, holding n_in and n_out");
+    return NGPU_OK;
+}
+
+}  // namespace
+
+#define NGPU_TRY(x)                     \
+    do {                                \
+        const int rc_ = (x);            \
+        if (rc_ != NGPU_OK) return rc_; \
+    } while (0)
+
+extern "C" int64_t ngpu_mlp_workspace_bytes(int32_t M, int32_t width, int32_t k_in, int32_t n_out_p, int32_t train) {
+    if (M < 1 || width < 1 || k_in < 1 || n_out_p < 1) return 0;
+    Arena a{nullptr};
+    const int64_t Mp = pad_to(M, kGemmBM);
+    if (train) MlpTrainWs(a, Mp, width, k_in, n_out_p);
+    else MlpPredictWs(a, Mp, width, k_in, n_out_p);
+    return a.used;
+}
+
+extern "C" int ngpu_mlp_predict(const float* X, int32_t M, int32_t n_in, const float* x_mu, const float* x_sd,
+                                const void* const* wb, const float* const* b, int32_t width, int32_t k_in,
+                                int32_t n_out, int32_t n_out_p, const float* y_mu, const float* y_sd, void* ws,
+                                int64_t ws_bytes, float* out, void* cuda_stream) {
+    if (!X || !wb || !b || !ws || !out) return fail(NGPU_E_INVALID, "mlp_predict: null pointer");
+    NGPU_TRY(mlp_check(M, n_in, width, k_in, n_out, n_out_p));
+    const int Mp = (int)pad_to(M, kGemmBM), bn = width % 256 == 0 ? 256 : 128;
+    Arena a{(char*)ws};
+    const MlpPredictWs w(a, Mp, width, k_in, n_out_p);
+    if (ws_bytes < a.used) return fail(NGPU_E_INVALID, "mlp_predict: workspace too small");
+    cudaStream_t st = (cudaStream_t)cuda_stream;
+    k_mlp_input<<<dim3(Mp / 32, k_in / 32), 256, 0, st>>>(X, M, n_in, x_mu, x_sd, Mp, k_in, w.xb, nullptr);
+    const __nv_bfloat16* h = w.xb;
+    for (int k = 0; k < 3; ++k) {
+        __nv_bfloat16* o = k == 1 ? w.h1 : w.h0;
+        const int kk = k == 0 ? k_in : width;
+        NGPU_TRY(gemm_checked(h, wb[k], Mp, width, kk, kk, kk, kEpiGelu, bn, nullptr, o, nullptr, width, Mp, b[k],
+                              nullptr, st, kEpiGelu));
+        h = o;
+    }
+    NGPU_TRY(gemm_checked(h, wb[3], Mp, n_out_p, width, width, width, kEpiBias, 32, w.y, nullptr, nullptr, n_out_p, Mp,
+                          b[3], nullptr, st, kEpiGelu));
+    k_mlp_output<<<(unsigned)std::min<size_t>(((size_t)M * n_out + 255) / 256, 148 * 16), 256, 0, st>>>(w.y, M, n_out, n_out_p, y_mu, y_sd, out);
+    g_launches += 2;
+    NGPU_CUDA(cudaGetLastError());
+    return NGPU_OK;
+}
+
+extern "C" int ngpu_mlp_grads(const float* X, const float* Y, const float* weight, int32_t M, int32_t n_in,
+                              const float* x_mu, const float* x_sd, const float* y_mu, const float* y_sd,
+                              const void* const* wb, const void* const* wtb, const float* const* b, int32_t width,
+                              int32_t k_in, int32_t n_out, int32_t n_out_p, void* ws, int64_t ws_bytes, float* loss,
+                              float* const* gw, float* const* gb, void* cuda_stream) {
+    if (!X || !Y || !wb || !wtb || !b || !ws || !loss || !gw || !gb) return fail(NGPU_E_INVALID, "mlp_grads: null pointer");
+    NGPU_TRY(mlp_check(M, n_in, width, k_in, n_out, n_out_p));
+    if (n_out_p > 64) return fail(NGPU_E_INVALID, "mlp_grads: at most 64 outputs");
+    const int Mp = (int)pad_to(M, kGemmBM), bn = width % 256 == 0 ? 256 : 128;
+    Arena a{(char*)ws};
+    const MlpTrainWs w(a, Mp, width, k_in, n_out_p);
+    if (ws_bytes < a.used) return fail(NGPU_E_INVALID, "mlp_grads: workspace too small");
+    cudaStream_t st = (cudaStream_t)cuda_stream;
+    k_mlp_input<<<dim3(Mp / 32, k_in / 32), 256, 0, st>>>(X, M, n_in, x_mu, x_sd, Mp, k_in, w.xb, w.ht[0]);
+    const __nv_bfloat16* h = w.xb;
+    for (int k = 0; k < 3; ++k) {
+        const int kk = k == 0 ? k_in : width;
+        NGPU_TRY(gemm_checked(h, wb[k], Mp, width, kk, kk, kk, kEpiBiasGelu, bn, w.z[k], w.h[k], w.ht[k + 1], width, Mp,
+                              b[k], nullptr, st, kEpiGelu));
+        h = w.h[k];
+    }
+    NGPU_TRY(gemm_checked(h, wb[3], Mp, n_out_p, width, width, width, kEpiBias, 32, w.y, nullptr, nullptr, n_out_p, Mp,
+                          b[3], nullptr, st, kEpiGelu));
+    NGPU_CUDA(cudaMemsetAsync(w.done, 0, sizeof(unsigned), st));
+    const MlpLossArgs la{w.y, Y, y_mu, y_sd, weight, M, Mp, n_out, n_out_p, w.dyb, w.dybt, w.part, w.done, loss, gb[3]};
+    k_mlp_loss<<<(Mp + kMlpLossRows - 1) / kMlpLossRows, 256, 0, st>>>(la);
+    // output layer: dW^T[width][n_out_p] = H^T dY
+    NGPU_TRY(gemm_checked(w.ht[3], w.dybt, width, n_out_p, Mp, Mp, Mp, kEpiSplitAdd, 32, w.g4t, nullptr, nullptr,
+                          n_out_p, width, nullptr, nullptr, st, kEpiGelu));
+    k_mlp_transpose<<<dim3((width + 31) / 32, n_out_p / 32), 256, 0, st>>>(w.g4t, width, n_out_p, gw[3]);
+    const __nv_bfloat16* dz = w.dyb;
+    for (int k = 2; k >= 0; --k) {
+        const int kd = k == 2 ? 64 : width, kin = k == 0 ? k_in : width;
+        NGPU_TRY(gemm_checked(dz, wtb[k + 1], Mp, width, kd, kd, kd, kEpiGeluGrad, bn, nullptr, w.dzb[k], w.dzbt[k],
+                              width, Mp, nullptr, w.z[k], st, kEpiGelu));
+        NGPU_TRY(gemm_checked(w.dzbt[k], w.ht[k], width, kin, Mp, Mp, Mp, kEpiSplitAdd, kin == 64 ? 64 : 128,
+                              gw[k], nullptr, nullptr, kin, width, nullptr, nullptr, st, kEpiGelu));
+        dz = w.dzb[k];
+    }
+    const MlpBiasArgs ba{{w.dzbt[0], w.dzbt[1], w.dzbt[2]}, {gb[0], gb[1], gb[2]}, Mp};
+    k_mlp_bias_grads<<<dim3(width, 3), 128, 0, st>>>(ba);
+    g_launches += 4;
+    NGPU_CUDA(cudaGetLastError());
+    return NGPU_OK;
+}
+
+extern "C" int ngpu_mlp_adam(float* const* p, const float* const* g, float* const* m, float* const* v, void* const* wb,
+                             void* const* wtb, int32_t n_in, int32_t width, int32_t k_in, int32_t n_out,
+                             int32_t n_out_p, float lr, float b1, float b2, float eps, float c1, float c2,
+                             void* cuda_stream) {
+    if (!p || !g || !m || !v || !wb || !wtb) return fail(NGPU_E_INVALID, "mlp_adam: null pointer");
+    NGPU_TRY(mlp_check(1, n_in, width, k_in, n_out, n_out_p));
+    MlpAdamArgs a;
+    const int rows[8] = {width, width, width, n_out_p, 1, 1, 1, 1};
+    const int cols[8] = {k_in, width, width, width, width, width, width, n_out_p};
+    a.tile0[0] = 0;
+    for (int k = 0; k < 8; ++k) {
+        if (!p[k] || !g[k] || !m[k] || !v[k] || (k < 4 && (!wb[k] || !wtb[k])))
+            return fail(NGPU_E_INVALID, "mlp_adam: null tensor");
+        a.p[k] = p[k], a.g[k] = g[k], a.m[k] = m[k], a.v[k] = v[k];
+        a.rows[k] = rows[k], a.cols[k] = cols[k];
+        if (k < 4) {
+            a.wb[k] = (__nv_bfloat16*)wb[k], a.wtb[k] = (__nv_bfloat16*)wtb[k];
+            a.ldt[k] = k == 3 ? 64 : rows[k];
+        }
+        a.tile0[k + 1] = a.tile0[k] + (k < 4 ? ((rows[k] + 31) / 32) * ((cols[k] + 31) / 32) : (cols[k] + 1023) / 1024);
+    }
+    a.n_in = n_in, a.n_out = n_out;
+    a.lr = lr, a.b1 = b1, a.b2 = b2, a.eps = eps, a.c1 = c1, a.c2 = c2;
+    k_mlp_adam<<<a.tile0[8], 256, 0, (cudaStream_t)cuda_stream>>>(a);
+    g_launches++;
+    NGPU_CUDA(cudaGetLastError());
     return NGPU_OK;
 }
 

@@ -2,16 +2,17 @@
 
 A 4-layer MLP (in -> 512 -> 512 -> 512 -> out, GELU in its tanh form) whose
 forward and backward products all run on the project's tcgen05 BF16 GEMM
-(ngpu_gemm_bf16_tn, FP32 accumulation in tensor memory) with fused
-epilogues:
-  forward   Z = H W^T + b, H' = gelu(Z)      (epilogue 1: Z fp32, H' bf16 and
-                                              its transpose for the weight
-                                              gradients)
-  output    Y = H W^T + b                    (epilogue 2)
-  backward  dZ = (dZ_next W) * gelu'(Z)      (epilogue 3, bf16 + transpose)
-            dW = dZ^T H                      (epilogue 0, K = the batch)
-PyTorch holds the buffers and does the elementwise optimizer step (Adam on
-FP32 master weights) and the bias sums; it does no matrix products.
+(FP32 accumulation in tensor memory) with fused epilogues:
+  forward   Z = H W^T + b, H' = gelu(Z)      (Z fp32, H' bf16 and its transpose
+                                              for the weight gradients; a
+                                              prediction writes H' alone)
+  output    Y = H W^T + b
+  backward  dZ = (dZ_next W) * gelu'(Z)      (bf16 + transpose)
+            dW = dZ^T H                      (K, the batch, split over CTAs)
+Operand preparation, the loss, bias gradients and the Adam step (FP32 master
+weights and their bf16 copies) are kernels of their own (csrc/mlp.cuh); each
+of predict, loss_and_grads and adam_step is one library call.  PyTorch holds
+the buffers.
 
 Shapes are padded for the tensor cores: the input width to a multiple of 64,
 the output to 32, the batch to a multiple of 128 (padding rows carry zero
@@ -27,11 +28,16 @@ import numpy as np
 
 from . import _ffi
 
-EPI_STORE, EPI_BIAS_GELU, EPI_BIAS, EPI_GELU_GRAD, EPI_SPLIT = 0, 1, 2, 3, 4
-
-
 def _pad(n: int, m: int) -> int:
     return (n + m - 1) // m * m
+
+
+def _p(x):
+    return None if x is None else C.c_void_p(x.data_ptr())
+
+
+def _ptrs(xs):
+    return (C.c_void_p * len(xs))(*[x.data_ptr() for x in xs])
 
 
 class SurrogateMLP:
@@ -40,9 +46,6 @@ class SurrogateMLP:
         self.torch = torch
         self.dev = torch.device("cuda")
         self.n_in, self.n_out, self.width = n_in, n_out, width
-        # 256-wide tiles where the width allows: measured on B200 at batch 8192 x width 512,
-        # 0.020 ms per hidden-layer forward GEMM against 0.024 with 128-wide tiles
-        self.bn_hidden = 256 if width % 256 == 0 else 128
         self.k_in = _pad(n_in, 64)
         self.n_out_p = _pad(max(n_out, 16), 32)
         dims = [(width, self.k_in), (width, width), (width, width), (self.n_out_p, width)]
@@ -78,40 +81,24 @@ class SurrogateMLP:
                 wt = t.nn.functional.pad(wt, (0, 64 - self.n_out_p))
             self.Wtb.append(wt.to(t.bfloat16).contiguous())
 
-    def _gemm(self, A, B, M, N, K, epi, bn, out_f32=None, out_b=None, out_bt=None, ldo=None, ldt=None,
-              bias=None, zin=None):
-        p = lambda x: None if x is None else C.c_void_p(x.data_ptr())
-        st = C.c_void_p(self.torch.cuda.current_stream().cuda_stream)
-        _ffi.check("ngpu_gemm_bf16_tn", _ffi.lib().ngpu_gemm_bf16_tn(
-            p(A), p(B), M, N, K, A.shape[1], B.shape[1], epi, bn, p(out_f32), p(out_b), p(out_bt),
-            ldo if ldo is not None else N, ldt if ldt is not None else M, p(bias), p(zin), st))
-
-    def _prep_x(self, X):
+    def _f32(self, x, *shape):
+        """x as a contiguous float32 tensor of this shape on the network's device (broadcast as in arithmetic)."""
         t = self.torch
-        X = t.as_tensor(X, dtype=t.float32, device=self.dev)
-        M = X.shape[0]
-        Mp = _pad(M, 128)
-        xn = (X - self.x_mu) / self.x_sd if self.x_mu is not None else X
-        xb = t.zeros(Mp, self.k_in, device=self.dev, dtype=t.bfloat16)
-        xb[:M, :self.n_in] = xn.to(t.bfloat16)
-        return xb, M, Mp
+        return t.as_tensor(x, dtype=t.float32, device=self.dev).expand(*shape).contiguous()
 
-    def _forward(self, xb, Mp):
-        t = self.torch
-        W = self.width
-        acts = {"H0": xb, "H0t": xb.t().contiguous()}
-        h = xb
-        for k in range(3):
-            z = t.empty(Mp, W, device=self.dev)
-            hb = t.empty(Mp, W, device=self.dev, dtype=t.bfloat16)
-            hbt = t.empty(W, Mp, device=self.dev, dtype=t.bfloat16)
-            self._gemm(h, self.Wb[k], Mp, W, h.shape[1], EPI_BIAS_GELU, self.bn_hidden, z, hb, hbt, W, Mp,
-                       bias=self.b[k])
-            acts[f"Z{k + 1}"], acts[f"H{k + 1}"], acts[f"H{k + 1}t"] = z, hb, hbt
-            h = hb
-        y = t.empty(Mp, self.n_out_p, device=self.dev)
-        self._gemm(h, self.Wb[3], Mp, self.n_out_p, W, EPI_BIAS, 32, y, bias=self.b[3])
-        return y, acts
+    def _stats(self, mu, sd, n):
+        """(keeps, pointer, pointer) of standardisation vectors, or of none."""
+        if mu is None:
+            return (), None, None
+        m, s = self._f32(mu, n), self._f32(sd, n)
+        return (m, s), _p(m), _p(s)
+
+    def _workspace(self, M, train):
+        n = int(_ffi.lib().ngpu_mlp_workspace_bytes(M, self.width, self.k_in, self.n_out_p, int(train)))
+        return self.torch.empty(max(n, 1), dtype=self.torch.uint8, device=self.dev), n
+
+    def _stream(self):
+        return C.c_void_p(self.torch.cuda.current_stream().cuda_stream)
 
     # ------------------------------------------------------------------- API
     def fit_stats(self, X, Y):
@@ -123,47 +110,37 @@ class SurrogateMLP:
 
     def predict(self, X):
         """Features (original units) for inputs X [M, n_in]."""
-        xb, M, Mp = self._prep_x(X)
-        y, _ = self._forward(xb, Mp)
-        out = y[:M, :self.n_out]
-        return out * self.y_sd + self.y_mu if self.y_mu is not None else out
+        t = self.torch
+        X = t.as_tensor(X, dtype=t.float32, device=self.dev)
+        M = X.shape[0]
+        X = self._f32(X, M, self.n_in)
+        out = t.empty(M, self.n_out, device=self.dev)
+        ws, n = self._workspace(M, False)
+        kx, x_mu, x_sd = self._stats(self.x_mu, self.x_sd, self.n_in)
+        ky, y_mu, y_sd = self._stats(self.y_mu, self.y_sd, self.n_out)
+        _ffi.check("ngpu_mlp_predict", _ffi.lib().ngpu_mlp_predict(
+            _p(X), M, self.n_in, x_mu, x_sd, _ptrs(self.Wb), _ptrs(self.b), self.width, self.k_in, self.n_out,
+            self.n_out_p, y_mu, y_sd, _p(ws), n, _p(out), self._stream()))
+        return out
 
     def loss_and_grads(self, X, Y, weight=None):
         """Mean squared error on standardised targets and the gradients of
         every weight and bias (lists in layer order)."""
         t = self.torch
-        xb, M, Mp = self._prep_x(X)
-        Yt = t.as_tensor(Y, dtype=t.float32, device=self.dev)
-        yn = (Yt - self.y_mu) / self.y_sd if self.y_mu is not None else Yt
-        y, a = self._forward(xb, Mp)
-        diff = y[:M, :self.n_out] - yn
+        X = t.as_tensor(X, dtype=t.float32, device=self.dev)
+        M = X.shape[0]
+        X, Y = self._f32(X, M, self.n_in), self._f32(Y, M, self.n_out)
         if weight is not None:
-            diff = diff * t.as_tensor(weight, dtype=t.float32, device=self.dev)[:, None]
-        count = M * self.n_out
-        loss = (diff * diff).sum() / count
-        dy = t.zeros(Mp, 64, device=self.dev)
-        dy[:M, :self.n_out] = 2.0 * diff / count
-        dyb = dy.to(t.bfloat16).contiguous()
-        dybt = dyb[:, :self.n_out_p].t().contiguous()          # [n_out_p][Mp]
-        W = self.width
-        gW, gb = [None] * 4, [None] * 4
-        # output layer: dW4^T[W][n_out_p] = H3^T . dY  (A = H3^T [W][Mp], B = dY^T [n_out_p][Mp])
-        g4t = t.empty(W, self.n_out_p, device=self.dev)
-        self._gemm(a["H3t"], dybt, W, self.n_out_p, Mp, EPI_SPLIT, 32, g4t)
-        gW[3] = g4t.t().contiguous()
-        gb[3] = dy[:, :self.n_out_p].sum(0)
-        dz = dyb
-        wt = self.Wtb[3]
-        for k in (2, 1, 0):                      # layer k+1 (1-based)
-            dzb = t.empty(Mp, W, device=self.dev, dtype=t.bfloat16)
-            dzbt = t.empty(W, Mp, device=self.dev, dtype=t.bfloat16)
-            self._gemm(dz, wt, Mp, W, dz.shape[1], EPI_GELU_GRAD, self.bn_hidden, None, dzb, dzbt, W, Mp,
-                       zin=a[f"Z{k + 1}"])
-            kin = self.k_in if k == 0 else W
-            g = t.empty(W, kin, device=self.dev)
-            self._gemm(dzbt, a[f"H{k}t"], W, kin, Mp, EPI_SPLIT, 64 if kin == 64 else 128, g)
-            gW[k], gb[k] = g, dzb.float().sum(0)
-            dz, wt = dzb, self.Wtb[k]
+            weight = self._f32(weight, M)
+        ws, n = self._workspace(M, True)
+        kx, x_mu, x_sd = self._stats(self.x_mu, self.x_sd, self.n_in)
+        ky, y_mu, y_sd = self._stats(self.y_mu, self.y_sd, self.n_out)
+        loss = t.empty((), device=self.dev)
+        gW, gb = [t.empty(w.shape, device=self.dev) for w in self.W], [t.empty(b.shape, device=self.dev) for b in self.b]
+        _ffi.check("ngpu_mlp_grads", _ffi.lib().ngpu_mlp_grads(
+            _p(X), _p(Y), _p(weight), M, self.n_in, x_mu, x_sd, y_mu, y_sd, _ptrs(self.Wb), _ptrs(self.Wtb),
+            _ptrs(self.b), self.width, self.k_in, self.n_out, self.n_out_p, _p(ws), n, _p(loss), _ptrs(gW), _ptrs(gb),
+            self._stream()))
         return loss, gW, gb
 
     def adam_step(self, gW, gb, lr=None, b1=0.9, b2=0.999, eps=1e-8):
@@ -171,16 +148,21 @@ class SurrogateMLP:
         lr = self.lr if lr is None else lr
         self.step_n += 1
         params = self.W + self.b
-        grads = gW + gb
-        c1, c2 = 1 - b1 ** self.step_n, 1 - b2 ** self.step_n
-        for p, g, m, v in zip(params, grads, self.m, self.v):
-            m.mul_(b1).add_(g, alpha=1 - b1)
-            v.mul_(b2).addcmul_(g, g, value=1 - b2)
-            p.addcdiv_(m / c1, (v / c2).sqrt_().add_(eps), value=-lr)
-        self.W[0][:, self.n_in:] = 0.0
-        self.W[3][self.n_out:, :] = 0.0
-        self.b[3][self.n_out:] = 0.0
-        self._refresh()
+        grads = [self._f32(g, *p.shape) for g, p in zip(list(gW) + list(gb), params)]
+        plain = lambda x: x if x.is_cuda and x.dtype == t.float32 and x.is_contiguous() else self._f32(x, *x.shape)
+        state = [[plain(x) for x in xs] for xs in (params, self.m, self.v)]
+        wb = [t.empty(w.shape, device=self.dev, dtype=t.bfloat16) for w in self.W]
+        wtb = [t.empty((w.shape[1], 64 if k == 3 else w.shape[0]), device=self.dev, dtype=t.bfloat16)
+               for k, w in enumerate(self.W)]
+        _ffi.check("ngpu_mlp_adam", _ffi.lib().ngpu_mlp_adam(
+            _ptrs(state[0]), _ptrs(grads), _ptrs(state[1]), _ptrs(state[2]), _ptrs(wb), _ptrs(wtb), self.n_in,
+            self.width, self.k_in, self.n_out, self.n_out_p, float(lr), float(b1), float(b2), float(eps),
+            1 - b1 ** self.step_n, 1 - b2 ** self.step_n, self._stream()))
+        for xs, ys in zip((params, self.m, self.v), state):
+            for x, y in zip(xs, ys):
+                if x is not y:
+                    x.copy_(y)
+        self.Wb, self.Wtb = wb, wtb
 
     def train(self, X, Y, epochs: int = 10, batch: int = 4096, lr: float | None = None, seed: int = 0,
               X_val=None, Y_val=None) -> list[float]:
