@@ -416,8 +416,8 @@ int ngpu_mlp_grads(const float *X, const float *Y, const float *weight, int32_t 
                    int32_t n_out_p, void *ws, int64_t ws_bytes, float *loss, float *const *gw, float *const *gb,
                    void *cuda_stream);
 int ngpu_mlp_adam(float *const *p, const float *const *g, float *const *m, float *const *v, void *const *wb,
-                  void *const *wtb, int32_t n_in, int32_t width, int32_t k_in, int32_t n_out, int32_t n_out_p, float lr,
-                  float b1, float b2, float eps, float c1, float c2, void *cuda_stream);
+                  void *const *wtb, int32_t n_in, int32_t width, int32_t k_in, int32_t n_out, int32_t n_out_p,
+                  double lr, double b1, double b2, double eps, double c1, double c2, void *cuda_stream);
 
 /*
  * Genetic-algorithm steps on the device (all pointers device memory, all

@@ -71,7 +71,7 @@ def lib() -> C.CDLL:
             "ngpu_mlp_predict": (C.c_int, [P, I32, I32, P, P, P, P, I32, I32, I32, I32, P, P, P, I64, P, P]),
             "ngpu_mlp_grads": (C.c_int, [P, P, P, I32, I32, P, P, P, P, P, P, P, I32, I32, I32, I32, P, I64, P, P, P,
                                          P]),
-            "ngpu_mlp_adam": (C.c_int, [P, P, P, P, P, P, I32, I32, I32, I32, I32, F32, F32, F32, F32, F32, F32, P]),
+            "ngpu_mlp_adam": (C.c_int, [P, P, P, P, P, P, I32, I32, I32, I32, I32, D, D, D, D, D, D, P]),
             "ngpu_sim_destroy": (C.c_int, [P]),
             "ngpu_sim_set_params": (C.c_int, [P, P, I32]),
             "ngpu_sim_set_stimulus": (C.c_int, [P, I32, P, P, I32, F32, I32]),

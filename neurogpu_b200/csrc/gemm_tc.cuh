@@ -175,8 +175,6 @@ __device__ __forceinline__ void epi_one(const GemmArgs& g, float* sp, size_t o, 
         g.out_f32[o] = d + g.bias[n];
     } else if constexpr (EPI == kEpiSplitAdd) {
         atomicAdd(g.out_f32 + o, d);
-    } else if constexpr (EPI == kEpiGelu) {
-        g.out_bf16[o] = __float2bfloat16_rn(gelu_tanh(d + g.bias[n]));
     } else if constexpr (EPI == kEpiBiasGelu) {
         const float z = d + g.bias[n];
         const __nv_bfloat16 h = __float2bfloat16_rn(gelu_tanh(z));
@@ -204,11 +202,10 @@ __device__ __forceinline__ void epi_vec4(const GemmArgs& g, float* sp, size_t o,
         *reinterpret_cast<float4*>(g.out_f32 + o) = make_float4(d[0], d[1], d[2], d[3]);
     } else {
         float v[4];
-        if constexpr (EPI == kEpiBiasGelu || EPI == kEpiGelu) {
+        if constexpr (EPI == kEpiBiasGelu) {
             const float4 b = *reinterpret_cast<const float4*>(g.bias + n);
             const float z[4] = {d[0] + b.x, d[1] + b.y, d[2] + b.z, d[3] + b.w};
-            if constexpr (EPI == kEpiBiasGelu)
-                *reinterpret_cast<float4*>(g.out_f32 + o) = make_float4(z[0], z[1], z[2], z[3]);
+            *reinterpret_cast<float4*>(g.out_f32 + o) = make_float4(z[0], z[1], z[2], z[3]);
 #pragma unroll
             for (int q = 0; q < 4; ++q) v[q] = gelu_tanh(z[q]);
         } else {  // kEpiGeluGrad
@@ -221,8 +218,7 @@ __device__ __forceinline__ void epi_vec4(const GemmArgs& g, float* sp, size_t o,
         pk.x = *reinterpret_cast<const uint32_t*>(&lo);
         pk.y = *reinterpret_cast<const uint32_t*>(&hi);
         *reinterpret_cast<uint2*>(g.out_bf16 + o) = pk;
-        if constexpr (EPI != kEpiGelu)
-            sp[0] = __low2float(lo), sp[1] = __high2float(lo), sp[2] = __low2float(hi), sp[3] = __high2float(hi);
+        sp[0] = __low2float(lo), sp[1] = __high2float(lo), sp[2] = __low2float(hi), sp[3] = __high2float(hi);
     }
 }
 
@@ -234,9 +230,67 @@ __device__ __forceinline__ void epi_vec4(const GemmArgs& g, float* sp, size_t o,
 // outputs with coalesced stores (see GemmEpilogue).  Any four consecutive
 // warps cover the four quarters, so the group w0 + 4k .. w0 + 4k + 3 takes
 // slice k whatever w0 is.  Warps past the last slice have no work.
+// The activations-only epilogue needs no staging: a lane holds 32 columns of
+// its row, 64 bytes of bf16, and writes them as whole 16-byte vectors.  24,576
+// x 512 x 512: 31 us staged (8 warps' dependent instructions, 10 us a tile
+// against 3 us of MMAs).
+__device__ __forceinline__ void gelu_epilogue_row(const GemmArgs& g, const uint32_t (&r)[32], int m, int n) {
+    if (m >= g.M) return;
+    const size_t o = (size_t)m * g.ldo + n;
+    if (n + 32 <= g.N && g.ldo % 8 == 0 && (((uintptr_t)g.out_bf16 | (uintptr_t)g.bias) & 15) == 0) {
+#pragma unroll
+        for (int c = 0; c < 32; c += 8) {
+            const float4 b0 = *reinterpret_cast<const float4*>(g.bias + n + c);
+            const float4 b1 = *reinterpret_cast<const float4*>(g.bias + n + c + 4);
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            uint32_t h[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const __nv_bfloat162 v = __floats2bfloat162_rn(gelu_tanh(__uint_as_float(r[c + 2 * q]) + b[2 * q]),
+                                                               gelu_tanh(__uint_as_float(r[c + 2 * q + 1]) + b[2 * q + 1]));
+                h[q] = *reinterpret_cast<const uint32_t*>(&v);
+            }
+            *reinterpret_cast<uint4*>(g.out_bf16 + o + c) = make_uint4(h[0], h[1], h[2], h[3]);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+            if (n + c < g.N) g.out_bf16[o + c] = __float2bfloat16_rn(gelu_tanh(__uint_as_float(r[c]) + g.bias[n + c]));
+    }
+}
+
+template <int BN, int NW>
+__device__ __forceinline__ void gelu_epilogue(const GemmArgs& g, uint32_t tmem, int m0, int n0, int w0) {
+    constexpr int kSlices = (NW / 4) < (BN / 32) ? (NW / 4) : (BN / 32);
+    constexpr int kCols = BN / kSlices;  // a multiple of 32
+    static_assert(NW % 4 == 0 && kCols % 32 == 0, "epilogue slices");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q = warp & 3, slice = (warp - w0) >> 2;
+    if (slice >= kSlices) return;
+    const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+#pragma unroll 1
+    for (int c0 = slice * kCols; c0 < (slice + 1) * kCols; c0 += 32) {
+        uint32_t r[32];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+              "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+            : "r"(trow + (uint32_t)c0));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        gelu_epilogue_row(g, r, m0 + q * 32 + lane, n0 + c0);
+    }
+}
+
 template <int BN, int EPI, int NW = 4>
 __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, uint32_t tmem, float* stage, int m0, int n0,
                                               int w0 = 0) {
+    if constexpr (EPI == kEpiGelu) {
+        gelu_epilogue<BN, NW>(g, tmem, m0, n0, w0);
+        return;
+    }
     constexpr int kSlices = (NW / 4) < (BN / 16) ? (NW / 4) : (BN / 16);
     constexpr int kCols = BN / kSlices;  // a multiple of 16
     static_assert(NW % 4 == 0 && kCols % 16 == 0, "epilogue slices");
@@ -567,8 +621,10 @@ __global__ void __launch_bounds__(kTmaThreads) k_gemm_bf16_tma(const __grid_cons
 // at the same time share operand tiles in L2.  Every wait is bounded; a role
 // whose wait gives up records the error and stops, and the others' waits
 // then run out in turn.
-constexpr int kPersistThreads = 10 * 32;
 constexpr int kPersistEpiWarps = 8;  // overlapped with the MMAs, so fewer warps suffice; the ring keeps 4-8 stages
+// The activations-only epilogue stages nothing, so 16 warps cost no ring stage.
+__host__ __device__ constexpr int persist_epi_warps(int epi) { return epi == kEpiGelu ? 16 : kPersistEpiWarps; }
+__host__ __device__ constexpr int persist_threads(int epi) { return (2 + persist_epi_warps(epi)) * 32; }
 constexpr int kPersistGroupM = 16;
 
 template <int BN>
@@ -602,7 +658,7 @@ __device__ __forceinline__ void persist_unit(int u, int n_mt, int n_nt, int& mt,
 }
 
 template <int BN, int EPI>
-__global__ void __launch_bounds__(kPersistThreads, 1)
+__global__ void __launch_bounds__(persist_threads(EPI), 1)
     k_gemm_bf16_tma_persistent(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                                GemmArgs g, int n_units, int n_mt, int n_nt) {
     static_assert(BN % 16 == 0 && BN >= 32 && BN <= 256, "BN: a multiple of 16 in [32, 256]");
@@ -628,7 +684,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&Sm.tfull[b]), 1);
-            mbar_init(smem_u32(&Sm.tempty[b]), kPersistEpiWarps);
+            mbar_init(smem_u32(&Sm.tempty[b]), persist_epi_warps(EPI));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tma_a) : "memory");
@@ -696,7 +752,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
                              : "memory");
             }
         }
-    } else {  // epilogue warps 2 .. 9
+    } else {  // epilogue warps 2 .. 9 (17)
         uint32_t t = 0;
         for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++t) {
             int mt, nt, z;
@@ -705,7 +761,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
             ok = mbar_wait(smem_u32(&Sm.tfull[b]), j & 1u);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            gemm_epilogue<BN, EPI, kPersistEpiWarps>(g, tmem + b * (uint32_t)BN, Sm.stage, mt * kGemmBM, nt * BN,
+            gemm_epilogue<BN, EPI, persist_epi_warps(EPI)>(g, tmem + b * (uint32_t)BN, Sm.stage, mt * kGemmBM, nt * BN,
                                                      2);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();

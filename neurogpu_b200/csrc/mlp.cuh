@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256) k_mlp_output(const float* y, int M, int n
 
 // Loss and its gradient at the output: diff = (y - target) * weight, target
 // standardised; dy = 2 diff / count as bf16, row-major [Mp][64] (zero past
-// n_out columns and M rows) and transposed [n_out_p][Mp].  A CTA per 64 rows
+// n_out columns and M rows) and transposed [n_out_p][Mp].  A CTA per 32 rows
 // leaves its sum of diff^2 and its column sums of dy in part[block][1 +
 // n_out_p]; the last CTA to finish adds them up in block order.
 struct MlpLossArgs {
@@ -70,7 +70,7 @@ struct MlpLossArgs {
     float* loss;
     float* gb;               // [n_out_p]
 };
-constexpr int kMlpLossRows = 64;
+constexpr int kMlpLossRows = 32;
 __global__ void __launch_bounds__(256) k_mlp_loss(const MlpLossArgs a) {
     __shared__ float d_s[kMlpLossRows][65];
     __shared__ float sq_s[8];
@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(256) k_mlp_loss(const MlpLossArgs a) {
     const int m0 = blockIdx.x * kMlpLossRows;
     const float count = (float)((int64_t)a.M * a.n_out);
     float sq = 0.f;
+#pragma unroll
     for (int t = threadIdx.x; t < kMlpLossRows * 64; t += 256) {
         const int r = t >> 6, c = t & 63, m = m0 + r;
         float dy = 0.f;
@@ -113,10 +114,18 @@ __global__ void __launch_bounds__(256) k_mlp_loss(const MlpLossArgs a) {
     if (threadIdx.x == 0) last = atomicAdd(a.done, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
-    for (int c = threadIdx.x; c < np; c += 256) {
+    // four threads per sum, each every fourth block (np <= 65)
+    __shared__ double sum_s[4][65];
+    for (int t = threadIdx.x; t < 4 * np; t += 256) {
+        const int c = t % np, q = t / np;
         double s = 0.0;
 #pragma unroll 8
-        for (unsigned b = 0; b < gridDim.x; ++b) s += (double)__ldcg(a.part + (size_t)b * np + c);
+        for (unsigned b = q; b < gridDim.x; b += 4) s += (double)__ldcg(a.part + (size_t)b * np + c);
+        sum_s[q][c] = s;
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < np; c += 256) {
+        const double s = (sum_s[0][c] + sum_s[1][c]) + (sum_s[2][c] + sum_s[3][c]);
         if (c == 0) *a.loss = __fdiv_rn((float)s, count);
         else a.gb[c - 1] = (float)s;
     }
@@ -171,12 +180,12 @@ struct MlpAdamArgs {
     int ldt[4];              // columns of the transposed copy
     int tile0[9];            // first CTA of each tensor
     int n_in, n_out;
-    float lr, b1, b2, eps, c1, c2;
+    float lr, b1, b2, d1, d2, eps, c1, c2;  // d1 = 1 - b1, d2 = 1 - b2 (rounded once each)
 };
 __device__ __forceinline__ float mlp_adam(const MlpAdamArgs& a, int k, size_t o, bool keep) {
     const float g = a.g[k][o];
-    const float m = fmaf(1.0f - a.b1, g, a.m[k][o] * a.b1);
-    const float v = fmaf((1.0f - a.b2) * g, g, a.v[k][o] * a.b2);
+    const float m = fmaf(a.d1, g, a.m[k][o] * a.b1);
+    const float v = fmaf(a.d2 * g, g, a.v[k][o] * a.b2);
     a.m[k][o] = m;
     a.v[k][o] = v;
     float p = a.p[k][o] - a.lr * __fdiv_rn(__fdiv_rn(m, a.c1), __fadd_rn(__fsqrt_rn(__fdiv_rn(v, a.c2)), a.eps));

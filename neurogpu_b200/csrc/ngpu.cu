@@ -2670,7 +2670,7 @@ static cudaError_t launch_gemm_bn(GemmArgs g, cudaStream_t st) {
                     if (e != cudaSuccess) return e;
                 }
                 const int units = n_mt * n_nt * splits;
-                k_gemm_bf16_tma_persistent<BN, EPI><<<std::min(units, kSmCount), kPersistThreads, smem, st>>>(
+                k_gemm_bf16_tma_persistent<BN, EPI><<<std::min(units, kSmCount), persist_threads(EPI), smem, st>>>(
                     ta, tb, g, units, n_mt, n_nt);
                 g_launches++;
                 return cudaGetLastError();
@@ -2810,6 +2810,13 @@ struct MlpTrainWs {
     }
 };
 
+// Column tile of the hidden layers: 256, unless 128-wide tiles still fit one
+// wave of SMs (4,096 rows x 512: 64 CTAs against 128; the epilogue sets their
+// time, 14-21 us a layer against 10-15).
+int mlp_tile(int Mp, int width) {
+    return width % 256 == 0 && (Mp / kGemmBM) * (width / 128) > kSmCount ? 256 : 128;
+}
+
 int mlp_check(int64_t M, int n_in, int width, int k_in, int n_out, int n_out_p) {
     if (M < 1 || M > (1 << 30)) return fail(NGPU_E_INVALID, "mlp: 1 <= rows <= 2^30");
     if (n_in < 1 || k_in < n_in || k_in % 64 || width < 64 || width % 64 || n_out < 1 || n_out_p < n_out ||
@@ -2841,7 +2848,7 @@ extern "C" int ngpu_mlp_predict(const float* X, int32_t M, int32_t n_in, const f
                                 int64_t ws_bytes, float* out, void* cuda_stream) {
     if (!X || !wb || !b || !ws || !out) return fail(NGPU_E_INVALID, "mlp_predict: null pointer");
     NGPU_TRY(mlp_check(M, n_in, width, k_in, n_out, n_out_p));
-    const int Mp = (int)pad_to(M, kGemmBM), bn = width % 256 == 0 ? 256 : 128;
+    const int Mp = (int)pad_to(M, kGemmBM), bn = mlp_tile(Mp, width);
     Arena a{(char*)ws};
     const MlpPredictWs w(a, Mp, width, k_in, n_out_p);
     if (ws_bytes < a.used) return fail(NGPU_E_INVALID, "mlp_predict: workspace too small");
@@ -2871,7 +2878,7 @@ extern "C" int ngpu_mlp_grads(const float* X, const float* Y, const float* weigh
     if (!X || !Y || !wb || !wtb || !b || !ws || !loss || !gw || !gb) return fail(NGPU_E_INVALID, "mlp_grads: null pointer");
     NGPU_TRY(mlp_check(M, n_in, width, k_in, n_out, n_out_p));
     if (n_out_p > 64) return fail(NGPU_E_INVALID, "mlp_grads: at most 64 outputs");
-    const int Mp = (int)pad_to(M, kGemmBM), bn = width % 256 == 0 ? 256 : 128;
+    const int Mp = (int)pad_to(M, kGemmBM), bn = mlp_tile(Mp, width);
     Arena a{(char*)ws};
     const MlpTrainWs w(a, Mp, width, k_in, n_out_p);
     if (ws_bytes < a.used) return fail(NGPU_E_INVALID, "mlp_grads: workspace too small");
@@ -2911,7 +2918,7 @@ extern "C" int ngpu_mlp_grads(const float* X, const float* Y, const float* weigh
 
 extern "C" int ngpu_mlp_adam(float* const* p, const float* const* g, float* const* m, float* const* v, void* const* wb,
                              void* const* wtb, int32_t n_in, int32_t width, int32_t k_in, int32_t n_out,
-                             int32_t n_out_p, float lr, float b1, float b2, float eps, float c1, float c2,
+                             int32_t n_out_p, double lr, double b1, double b2, double eps, double c1, double c2,
                              void* cuda_stream) {
     if (!p || !g || !m || !v || !wb || !wtb) return fail(NGPU_E_INVALID, "mlp_adam: null pointer");
     NGPU_TRY(mlp_check(1, n_in, width, k_in, n_out, n_out_p));
@@ -2931,7 +2938,8 @@ extern "C" int ngpu_mlp_adam(float* const* p, const float* const* g, float* cons
         a.tile0[k + 1] = a.tile0[k] + (k < 4 ? ((rows[k] + 31) / 32) * ((cols[k] + 31) / 32) : (cols[k] + 1023) / 1024);
     }
     a.n_in = n_in, a.n_out = n_out;
-    a.lr = lr, a.b1 = b1, a.b2 = b2, a.eps = eps, a.c1 = c1, a.c2 = c2;
+    a.lr = (float)lr, a.b1 = (float)b1, a.b2 = (float)b2, a.d1 = (float)(1.0 - b1), a.d2 = (float)(1.0 - b2);
+    a.eps = (float)eps, a.c1 = (float)c1, a.c2 = (float)c2;
     k_mlp_adam<<<a.tile0[8], 256, 0, (cudaStream_t)cuda_stream>>>(a);
     g_launches++;
     NGPU_CUDA(cudaGetLastError());
