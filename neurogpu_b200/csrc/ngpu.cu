@@ -490,6 +490,9 @@ struct ngpu_sim {
     DevSep* d_seps = nullptr;
     void* d_sepv = nullptr;
     int n_warps = 1;
+    bool warps_chosen = false;    // ... given by the caller
+    bool no_team = false;         // while a batch splits it
+    int ctas = 3;                 // CTAs per SM the batch is laid out for (kernels above 8 warps: compiled for)
     int team = 0;                 // CTAs (of n_warps warps) per group, one cluster; 0: one CTA per group
     int* d_skel = nullptr;        // the staged skeleton's tables (part.skel)
     int* d_team_items = nullptr;
@@ -536,11 +539,12 @@ struct ngpu_sim {
 
 // Work items per warp the tree is split into by default.  8-warp CTAs: 3
 // (ms per 200 steps at 12,288 instances with 1 / 2 / 3 / 4: TTPC-like 85.6 /
-// 83.6 / 77.6 / 83.3, HH 30.1 / 29.4 / 28.6 / 30.6).  Wide CTAs and teams: 1,
-// since a finer split lengthens the skeleton, which nothing hides there (us
-// per step with 1 / 2: HH cell, 33 instances 18.0 / 25.2; TTPC-like, 300
+// 83.6 / 77.6 / 83.3, HH 30.1 / 29.4 / 28.6 / 30.6).  12-warp CTAs: 2
+// (within 3 % of the best of 1 to 3 on four trees).  16-warp CTAs and teams:
+// 1, since a finer split lengthens the skeleton, which nothing hides there
+// (us per step with 1 / 2: HH cell, 33 instances 18.0 / 25.2; TTPC-like, 300
 // instances 33.4 / 40.6).
-static int default_items(int n_warps) { return n_warps > 8 ? 1 : 3; }
+static int default_items(int n_warps) { return n_warps > 12 ? 1 : n_warps > 8 ? 2 : 3; }
 
 // Thread-item layout: work items per instance at most / by default, and the
 // SM count the default CTA shape spreads a small batch over.
@@ -552,13 +556,31 @@ constexpr int kDefaultTiItems = 32;
 // Compartments per warp of a wide CTA: a passive cable of 50 takes 8.7 us per
 // step with 6 warps, 6.4 with 16; one of 128, 20 with 4 and 9.4 with 16.
 constexpr int kWideNodes = 3;
+// Compartments per warp of an 8-warp CTA.
+constexpr int kNarrowNodes = 16;
+// Warps a tree gets by default out of the `most` its CTA could have.
+static int default_warps(int n_nodes, int most) {
+    return std::min(most, std::max(1, n_nodes / (most > 8 ? kWideNodes : kNarrowNodes)));
+}
 constexpr int kSmCount = 148;
 
-// CTAs per SM that `smem` bytes of dynamic shared memory and W warps of 80
-// registers allow (228 KB per SM, 1 KB of it reserved per CTA).
-// CTAs per SM a wide (more than 8 warps) lane-instance kernel is compiled
-// for: 1 when the batch has at most one group per SM (registers are then
-// plentiful: 16 warps get 128), else 3 (one wave for large batches).
+// CTAs per SM that `smem` bytes of dynamic shared memory allow (228 KB per SM,
+// 1 KB of it reserved per CTA).
+static int ctas_by_smem(size_t smem) { return std::max(1, (int)((228 * 1024) / (smem + 1024))); }
+
+// CTAs per SM a batch of lane-instance groups is laid out for: three of 8
+// warps, fewer and wider ones where the groups or their shared memory do not
+// fill three (24 warps at 80 registers either way; one CTA per SM takes 16
+// warps at 128 registers).  Measured on B200, 160 groups, us per step with
+// 8-warp CTAs and with 12-warp ones: HH cells of 200 / 800 / 1500 / 3000
+// compartments 63 / 169 / 316 / 653 and 43 / 143 / 261 / 537; the four
+// together as one batch (two CTAs by shared memory) 860 and 760.
+static int resident_ctas(size_t smem_plain, int n_groups) {
+    return std::min({3, ctas_by_smem(smem_plain), (n_groups + kSmCount - 1) / kSmCount});
+}
+static int resident_warps(int ctas) { return ctas == 1 ? 16 : ctas == 2 ? 12 : 8; }
+
+// CTAs per SM that kernels for explicitly chosen wide CTAs are compiled for.
 static int wide_ctas_per_sm(int n_groups) { return n_groups <= kSmCount ? 1 : 3; }
 
 __global__ void k_cluster_probe() {}  // never launched: its occupancy is asked for
@@ -608,19 +630,13 @@ static int team_size(int n_groups, int n_nodes) {
     return 0;
 }
 
-static int ctas_per_sm(size_t smem, int W, int n_groups) {
-    // kernels of up to 8 warps use 80 registers; wider ones are compiled for wide_ctas_per_sm
-    const int by_regs = W > kMaxWarps ? wide_ctas_per_sm(n_groups) : 65536 / (kLanes * W * 80);
-    const int by_smem = (int)((228 * 1024) / (smem + 1024));
-    return std::max(1, std::min(std::min(by_regs, by_smem), 64 / W));
-}
-
-// Stage the skeleton in shared memory when that costs no occupancy.
+// Stage the skeleton in shared memory when that costs no occupancy (ctas: the
+// CTAs per SM the batch is laid out for).
 template <typename R>
-static int choose_s2_stage(int n_nodes, const Partition& P, int W, int n_groups) {
+static int choose_s2_stage(int n_nodes, const Partition& P, int W, int ctas) {
     if (W < 2 || P.seps.size() < 2) return 0;
     const size_t plain = lane_smem<R>(n_nodes, P, 0), staged = lane_smem<R>(n_nodes, P, 1);
-    return staged <= 227 * 1024 && ctas_per_sm(staged, W, n_groups) >= ctas_per_sm(plain, W, n_groups) ? 1 : 0;
+    return staged <= 227 * 1024 - 64 && ctas_by_smem(staged) >= std::min(ctas, ctas_by_smem(plain)) ? 1 : 0;
 }
 
 template <typename R>
@@ -1143,7 +1159,7 @@ static void sim_split_lanes(ngpu_sim* s) {
     const ngpu_model* m = s->m;
     const bool f8 = s->precision == NGPU_FP64;
     s->team = 0;
-    int team = s->n_warps > kMaxWarps ? team_size(s->n_groups, m->n) : 0;
+    int team = s->n_warps > kMaxWarps && s->ctas == 1 && !s->no_team ? team_size(s->n_groups, m->n) : 0;
     if (const char* ev = getenv("NGPU_TEAM")) team = std::min(team, atoi(ev));
     for (; team > 1; --team) {
         s->part = make_partition(m, s->n_warps * team, s->items_per_warp);
@@ -1155,10 +1171,18 @@ static void sim_split_lanes(ngpu_sim* s) {
             return;
         }
     }
+    // the library's item count gives way where the skeleton's rows would not
+    // fit beside it: unstaged, one warp walks them through memory (the
+    // TTPC-like cell at 12,288 instances: 0.40 ms per step staged, 0.58 not)
+    for (int k = s->items_per_warp; k >= 1; --k) {
+        s->part = make_partition(m, s->n_warps, k);
+        skeleton_tables(s->part);
+        s->s2_stage = f8 ? choose_s2_stage<double>(m->n, s->part, s->n_warps, s->ctas)
+                         : choose_s2_stage<float>(m->n, s->part, s->n_warps, s->ctas);
+        if (s->s2_stage || s->items_chosen || s->n_warps < 2) return;
+    }
     s->part = make_partition(m, s->n_warps, s->items_per_warp);
     skeleton_tables(s->part);
-    s->s2_stage = f8 ? choose_s2_stage<double>(m->n, s->part, s->n_warps, s->n_groups)
-                     : choose_s2_stage<float>(m->n, s->part, s->n_warps, s->n_groups);
 }
 
 // The device side of the simulation's tree split (s->part): junction
@@ -1258,13 +1282,20 @@ int ngpu_sim_create_layout(ngpu_model* m, int32_t n_sets, int32_t n_stim, int32_
     // warps per CTA and the tree split over them: a batch of at most one
     // 32-instance group per SM leaves SMs idle, so its CTAs get up to 16 warps
     // at one CTA per SM, and where SMs are still left a group gets a team of
-    // CTAs (sim_split_lanes); larger batches up to 8 (three CTAs per SM at 80
-    // registers)
-    int W = std::min(8, std::max(1, m->n / 48));
-    if (s->n_groups <= kSmCount && !ti && ngpu_jit::enabled() && ngpu_jit::nvrtc().ok)
-        W = std::min(kMaxWideWarps, std::max(1, m->n / kWideNodes));
-    if (const char* ev = getenv("NGPU_WARPS")) W = std::max(1, std::min(kMaxWideWarps, atoi(ev)));
-    if (n_warps > 0) W = n_warps;
+    // CTAs (sim_split_lanes); larger batches two CTAs of 12 or three of 8
+    const size_t plain = precision == NGPU_FP64 ? SmemPlan<double>::bytes(m->n) : SmemPlan<float>::bytes(m->n);
+    const bool wide = !ti && ngpu_jit::enabled() && ngpu_jit::nvrtc().ok;
+    s->ctas = wide ? resident_ctas(plain, s->n_groups) : std::min(3, ctas_by_smem(plain));
+    int W = default_warps(m->n, wide ? resident_warps(s->ctas) : kMaxWarps);
+    if (const char* ev = getenv("NGPU_WARPS")) {
+        W = std::max(1, std::min(kMaxWideWarps, atoi(ev)));
+        s->warps_chosen = true;
+    }
+    if (n_warps > 0) {
+        W = n_warps;
+        s->warps_chosen = true;
+    }
+    if (s->warps_chosen) s->ctas = W > kMaxWarps ? wide_ctas_per_sm(s->n_groups) : std::min(3, ctas_by_smem(plain));
     W = std::min(W, m->n);
     s->n_warps = W;
     s->items_per_warp = default_items(W);
@@ -1651,6 +1682,7 @@ int ngpu_sim_advance(ngpu_sim* s, int32_t t0, int32_t n_steps, void* cuda_stream
 struct ngpu_batch {
     std::vector<ngpu_sim*> sims;
     int precision = 0, mechset = 0, threads = 0, total_ctas = 0;
+    int ctas = 3;  // CTAs per SM it is laid out for
     size_t smem = 0;
     // a captured run (init + chunked advances), reused while its arguments hold
     cudaGraph_t graph = nullptr;
@@ -1709,7 +1741,7 @@ static int sim_upload_nodes(ngpu_sim* s) {
                                       s->folds, masks_cover(picked, all),
                                       s->layout == NGPU_LAYOUT_WARP_INSTANCE,
                                       s->layout == NGPU_LAYOUT_LANE_INSTANCE ? std::max(8, s->n_warps) : 8,
-                                      wide_ctas_per_sm(s->n_groups), s->team != 0);
+                                      s->ctas, s->team != 0);
         }
         if (gs && !s->jit)
             return fail(NGPU_E_CUDA, "mechanism set '" + gs->name +
@@ -1787,7 +1819,9 @@ static cudaError_t launch_batch(ngpu_batch* b, bool init, int t0, int n, cudaStr
     if (b->jit) {
         if (init) {
             void* args[] = {(void*)&B};
-            e = cudaLaunchKernel((const void*)b->jit->batch_init, dim3(b->total_ctas), dim3(b->threads), args, 0, st);
+            // (any warp count serves the init)
+            e = cudaLaunchKernel((const void*)b->jit->batch_init, dim3(b->total_ctas),
+                                 dim3(std::min(b->threads, kLanes * kMaxWarps)), args, 0, st);
         } else {
             const void* k = (const void*)b->jit->batch_advance;
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem);
@@ -1844,10 +1878,13 @@ static int batch_select_kernels(ngpu_batch* b) {
     }
     const std::vector<uint32_t> picked = ngpu_jit::pick_masks(all, kMaxClasses);
     b->jit = ngpu_jit::module(b->mechset, b->precision == NGPU_FP64, picked, gs ? &gs->source : nullptr,
-                              b->folds, masks_cover(picked, all));
+                              b->folds, masks_cover(picked, all), false, b->threads / kLanes, b->ctas);
     if (gs && !b->jit)
         return fail(NGPU_E_CUDA, "mechanism set '" + gs->name +
                                      "' runs only through runtime compilation: " + ngpu_jit::last_log());
+    if (!b->jit && b->threads > kLanes * kMaxWarps)
+        return fail(NGPU_E_CUDA, "CTAs of more than " + std::to_string(kMaxWarps) +
+                                     " warps run only through runtime compilation: " + ngpu_jit::last_log());
     return NGPU_OK;
 }
 
@@ -1870,16 +1907,30 @@ int ngpu_batch_create(ngpu_sim* const* sims, int32_t n, ngpu_batch** out) {
         if (sims[k]->layout != NGPU_LAYOUT_LANE_INSTANCE)
             return fail(NGPU_E_INVALID, "a batch holds lane-instance simulations only");
     }
-    // the batch kernel runs CTAs of up to kMaxWarps warps: a member created
-    // with wider CTAs (a small batch of its own) is split again for them
-    // and must be initialised again (through the batch)
+    // one launch, one CTA shape: members whose warps the library chose (or
+    // wider ones than 8) are split again for the CTAs per SM that the whole
+    // batch is laid out for, and must be initialised again (through the batch);
+    // a batch of at most one group per SM keeps CTAs of up to 8
+    const bool f8 = sims[0]->precision == NGPU_FP64;
+    size_t plain = 0;
+    int groups = 0;
+    for (int k = 0; k < n; ++k) {
+        plain = std::max(plain, f8 ? SmemPlan<double>::bytes(sims[k]->m->n) : SmemPlan<float>::bytes(sims[k]->m->n));
+        groups += sims[k]->n_groups;
+    }
+    const bool wide = groups > kSmCount && ngpu_jit::enabled() && ngpu_jit::nvrtc().ok;
+    const int ctas = wide ? resident_ctas(plain, groups) : std::min(3, ctas_by_smem(plain));
     for (int k = 0; k < n; ++k) {
         ngpu_sim* s = sims[k];
-        if (s->n_warps <= kMaxWarps) continue;
-        const int W = std::min(kMaxWarps, std::max(1, s->m->n / 48));
+        if (s->warps_chosen && s->n_warps <= kMaxWarps) continue;
+        const int W = default_warps(s->m->n, wide && !s->warps_chosen ? resident_warps(ctas) : kMaxWarps);
+        if (W == s->n_warps && !s->team && s->ctas == ctas) continue;
         s->n_warps = W;
+        s->ctas = ctas;
         if (!s->items_chosen) s->items_per_warp = default_items(W);
+        s->no_team = true;
         sim_split_lanes(s);
+        s->no_team = false;
         const int rc = sim_upload_split(s);
         if (rc != NGPU_OK) return rc;
         s->initialized = false;
@@ -1897,6 +1948,7 @@ int ngpu_batch_create(ngpu_sim* const* sims, int32_t n, ngpu_batch** out) {
                                                              : lane_smem<float>(s->m->n, s->part, s->s2_stage));
     }
     b->threads = kLanes * W;
+    b->ctas = ctas;
     b->folds = batch_common_folds(b);
     {
         const int rc = batch_select_kernels(b);
