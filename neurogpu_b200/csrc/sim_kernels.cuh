@@ -634,11 +634,6 @@ __global__ void __launch_bounds__(kLanes * kMaxWarps) k_sim_init(SimArgs<R> A) {
     init_body<R, MS>(A, blockIdx.x, &ctr);
 }
 
-// Back-substitution pass of an item, root -> leaf: the spine of a segment
-// (dV_i = r_i - c_i dV_parent + w_i dV_l, from separator u down), then the
-// light nodes; V update of each node.  Rows are prefetched into L2 in
-// blocks of four nodes, four nodes ahead.
-// TI: thread-item layout (lanes on different items; no lane-0 prefetch).
 // One node's back-substitution operands: its eliminated row (r, c; on a
 // spine also w) and its voltage with the Kahan term.
 template <typename R>
@@ -679,19 +674,27 @@ __device__ __forceinline__ void backsub_store(const SimArgs<R>& A, const Group<R
 // loaded before this node's update, so a node's memory latency overlaps the
 // previous node's arithmetic and stores (no node writes what the next one
 // reads: its own V and, for a junction, a dV its later children read).  Rows
-// are also prefetched into L2 in blocks of four nodes, four nodes ahead.
-// TI: thread-item layout (lanes on different items; no lane-0 prefetch).
-template <typename R, bool TI = false>
+// are also prefetched into L2 in blocks of four nodes, four nodes ahead, where
+// a grid of one CTA per group runs (148 groups, us per step without / with:
+// HH cell 80.9 / 72.9, TTPC-like 259 / 228).  Not with
+// TI: thread-item layout (lanes on different items; no lane-0 prefetch), and
+// not in FP32 with
+// TEAM: teams run on at most half the SMs, their rows stay in L2, and the
+// prefetch is instructions and a branch per block for nothing (without / with:
+// HH cell, 33 instances 17.5 / 18.0, 2,100 instances 29.0 / 30.1; TTPC-like,
+// 300 instances 32.6 / 34.0; in FP64 46.1 / 46.5 and 114 / 110, so FP64 keeps it).
+template <typename R, bool TI = false, bool TEAM = false>
 __device__ __forceinline__ void backsub_item(const SimArgs<R>& A, const Group<R>& G, const NodeRec<R>* nr,
                                              const DevComp& c, bool rec_now, float* trace, int& bad) {
     constexpr int kBlk = 4;
+    constexpr bool kAhead = !TI && !(TEAM && sizeof(R) == 4);
     if (c.l >= 0) {
         R xp = G.jx[(size_t)nr[c.u].jslot * kLanes];
         const R xl = G.jx[(size_t)nr[c.l].jslot * kLanes];
-        if constexpr (!TI) prefetch_backsub(G, c.r, min(kBlk, c.l - c.r));
+        if constexpr (kAhead) prefetch_backsub(G, c.r, min(kBlk, c.l - c.r));
         BackRow<R> cur = load_back_row<R, true>(G, c.r);
         for (int i = c.r; i < c.l; ++i) {
-            if constexpr (!TI)
+            if constexpr (kAhead)
                 if (((i - c.r) & (kBlk - 1)) == 0) prefetch_backsub(G, i + kBlk, min(kBlk, c.l - i - kBlk));
             const BackRow<R> nxt = i + 1 < c.l ? load_back_row<R, true>(G, i + 1) : cur;
             const R xi = cur.r - cur.c * xp + cur.w * xl;
@@ -702,12 +705,12 @@ __device__ __forceinline__ void backsub_item(const SimArgs<R>& A, const Group<R>
     }
     if (c.hi <= c.lo) return;
     R x_prev = 0;
-    if constexpr (!TI) prefetch_backsub(G, c.lo, min(kBlk, c.hi - c.lo));
+    if constexpr (kAhead) prefetch_backsub(G, c.lo, min(kBlk, c.hi - c.lo));
     NodeRec<R> n = nr[c.lo];
     BackRow<R> cur = load_back_row<R, false>(G, c.lo);
     R xj = n.pslot < 0 ? (R)0 : G.jx[(size_t)n.pslot * kLanes];
     for (int i = c.lo; i < c.hi; ++i) {
-        if constexpr (!TI)
+        if constexpr (kAhead)
             if (((i - c.lo) & (kBlk - 1)) == 0) prefetch_backsub(G, i + kBlk, min(kBlk, c.hi - i - kBlk));
         // the next node: its parent is this node (a chain child, pslot < 0)
         // or an earlier one, whose dV is already stored
@@ -959,7 +962,7 @@ __device__ __forceinline__ void run_item(const SimArgs<R>& A, const Group<R>& G,
     int lo = 0, hi = 0, sep = -1, sepk = k - A.n_comps, r = 0, lk = -1;
     if (k < A.n_comps) {
         const DevComp c = A.comps[k];
-        backsub_item<R, TI>(A, G, nr, c, rec_now, trace, bad);
+        backsub_item<R, TI, TEAM>(A, G, nr, c, rec_now, trace, bad);
         lo = c.lo;
         hi = c.hi;
         sep = c.l;
