@@ -38,7 +38,11 @@
 // differences within 2^-51 of each other, which samples with 2^-17 <= |v| <
 // 2^8 cannot have (their differences are exact multiples of 2^-40 below
 // 2^9).  Around any other sample (0, NaN, infinities, beyond 256 mV) the
-// quotients themselves are compared.
+// quotients themselves are compared.  Differences are compared as float32
+// first: rounding keeps their order, so where two round apart they are apart
+// that way, and where every |difference| is below every |v| they are exact
+// (the samples of a pair then lie within a factor of two).  Only a batch with
+// two equal rounded differences that may not be exact compares in float64.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -131,19 +135,30 @@ __host__ __device__ __forceinline__ void load_batch(const float* v, int64_t st, 
 }
 
 // Samples whose differences order as their quotients do: 2^-17 <= |v| < 2^8.
-// Collected from the bit patterns without the sign: the smallest and the
-// largest (infinities and NaN above every number).
+// The smallest and the largest |v|; a NaN fails the test.
 struct PlainRange {
-    uint32_t lo = 0xFFFFFFFFu, hi = 0;
-    __host__ __device__ __forceinline__ void add(float v) {
-        uint32_t b;
-        memcpy(&b, &v, 4);
-        b <<= 1;
-        lo = b < lo ? b : lo;
-        hi = b > hi ? b : hi;
+    float lo = INFINITY, hi = 0;
+    __host__ __device__ __forceinline__ void add(float a, float b) {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000  // (the tests' host build compiles for another)
+        asm("min.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(lo) : "f"(a), "f"(b));
+        asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(hi) : "f"(a), "f"(b));
+#else
+        lo = a != a || b != b ? 0 : fminf(lo, fminf(fabsf(a), fabsf(b)));
+        hi = fmaxf(hi, fmaxf(fabsf(a), fabsf(b)));
+#endif
     }
-    __host__ __device__ __forceinline__ bool ok() const { return lo >= (110u << 24) && hi < (135u << 24); }
+    __host__ __device__ __forceinline__ bool ok() const { return lo >= 0x1p-17f && hi < 0x1p8f; }
 };
+
+// The largest float32 that is not above x (a NaN stays one).
+__host__ __device__ __forceinline__ float float_below(double x) {
+#ifdef __CUDA_ARCH__
+    return __double2float_rd(x);
+#else
+    const float f = (float)x;
+    return (double)f > x ? nextafterf(f, -INFINITY) : f;
+#endif
+}
 
 // Steps 1 and 2 for the rises of trace t in [lo, hi) (lo a multiple of 8):
 // their peaks' positions go to rows lo / 2, lo / 2 + 1, ... of the scratch
@@ -164,60 +179,67 @@ __host__ __device__ inline int peaks_scan(const PeakArgs& a, int t, int lo, int 
     int m = 0, i0 = 0;
     if (j0 >= j1) return 0;
     bool up = false;
-    double vp = (double)v[(int64_t)j0 * st], dp = vp - (double)v[(int64_t)(j0 - 1) * st];
-    // sample j + 1 closes difference j
-    auto peak = [&](int j) {
-        if (dp / a.dt >= a.height) pos[(int64_t)m++ * ps] = (i0 + j - 1) / 2;
+    float xa = v[(int64_t)(j0 - 1) * st], xb = v[(int64_t)j0 * st];  // the two samples before the next
+    const float h_f = float_below(h_lo);
+    // sample j + 1 closes difference j; a fall from difference j - 1 = x1 - x0 ends a peak there
+    auto peak = [&](float x0, float x1, int j) {
+        if (((double)x1 - (double)x0) / a.dt >= a.height) pos[(int64_t)m++ * ps] = (i0 + j - 1) / 2;
     };
-    auto step = [&](float x, int j) {
-        const double vn = (double)x, d = vn - vp;
-        vp = vn;
-        const bool lt = dp < d, gt = d < dp;
-        if (up & gt & (dp >= h_lo)) peak(j);  // one predicate: a warp rarely goes in
-        up = lt | (up & !gt);
-        i0 = lt ? j : i0;
-        dp = d;
-    };
-    auto step_quotient = [&](float x, int j, bool may_rise) {
-        const double vn = (double)x, d = vn - vp, q = d / a.dt, qp = dp / a.dt;
-        vp = vn;
-        const bool lt = qp < q;
-        if (up && q < qp) peak(j);
-        up = lt ? may_rise : (up && q == qp);
+    auto step_exact = [&](float x, int j, bool quotient, bool may_rise) {
+        double d = (double)x - (double)xb, dp = (double)xb - (double)xa;
+        if (quotient) {
+            d /= a.dt;
+            dp /= a.dt;
+        }
+        const bool lt = dp < d;
+        if (up && d < dp) peak(xa, xb, j);
+        up = lt ? may_rise : (up && d == dp);
         if (lt) i0 = j;
-        dp = d;
+        xa = xb;
+        xb = x;
     };
     // samples j0 + 1 .. j1, in whole batches of 8 where they fit
     int s = j0 + 1;
-    for (; s <= j1 && (s & (kTraceBatch - 1)); ++s) step_quotient(v[(int64_t)s * st], s - 1, true);
+    for (; s <= j1 && (s & (kTraceBatch - 1)); ++s) step_exact(v[(int64_t)s * st], s - 1, true, true);
     if (s + kTraceBatch - 1 <= j1) {
-        PlainRange edge;  // the two samples before the first batch
-        edge.add(v[(int64_t)(s - 1) * st]);
-        edge.add(v[(int64_t)(s - 2) * st]);
-        bool plain_before = edge.ok() && !quotients;
         float nx8[kTraceBatch];
         load_batch(v, st, row, s, nx8);
         for (; s + kTraceBatch - 1 <= j1; s += kTraceBatch) {
-            float x[kTraceBatch];
-            PlainRange range;
+            float x[kTraceBatch + 2] = {xa, xb};
 #pragma unroll
-            for (int u = 0; u < kTraceBatch; ++u) {
-                x[u] = nx8[u];
-                range.add(x[u]);
-            }
+            for (int u = 0; u < kTraceBatch; ++u) x[u + 2] = nx8[u];
             if (s + 2 * kTraceBatch - 1 <= j1) load_batch(v, st, row, s + kTraceBatch, nx8);
-            const bool plain = range.ok() && !quotients;
-            if (plain && plain_before) {
+            PlainRange value, rise;
+            bool equal = false;
+            float d[kTraceBatch + 1];
 #pragma unroll
-                for (int u = 0; u < kTraceBatch; ++u) step(x[u], s + u - 1);
-            } else {
-                for (int u = 0; u < kTraceBatch; ++u) step_quotient(v[(int64_t)(s + u) * st], s + u - 1, true);
+            for (int u = 0; u <= kTraceBatch; ++u) {
+                d[u] = x[u + 1] - x[u];
+                if (u) equal = equal | (d[u] == d[u - 1]);
             }
-            plain_before = plain;
+#pragma unroll
+            for (int u = 0; u <= kTraceBatch; u += 2) {
+                value.add(x[u], x[u + 1]);
+                rise.add(d[u], d[u + 1 <= kTraceBatch ? u + 1 : u]);
+            }
+            const bool plain = value.ok() && !quotients;
+            if (plain && !(equal && !(rise.hi < value.lo))) {
+#pragma unroll
+                for (int u = 0; u < kTraceBatch; ++u) {
+                    const bool lt = d[u] < d[u + 1], gt = d[u + 1] < d[u];
+                    if (up & gt & (d[u] >= h_f)) peak(x[u], x[u + 1], s + u - 1);  // one predicate: a warp rarely goes in
+                    up = lt | (up & !gt);
+                    i0 = lt ? s + u - 1 : i0;
+                }
+                xa = x[kTraceBatch];
+                xb = x[kTraceBatch + 1];
+            } else {
+                for (int u = 0; u < kTraceBatch; ++u) step_exact(v[(int64_t)(s + u) * st], s + u - 1, !plain, true);
+            }
         }
     }
-    for (; s <= j1; ++s) step_quotient(v[(int64_t)s * st], s - 1, true);
-    for (; up && s <= nx; ++s) step_quotient(v[(int64_t)s * st], s - 1, false);  // only an open run goes on
+    for (; s <= j1; ++s) step_exact(v[(int64_t)s * st], s - 1, true, true);
+    for (; up && s <= nx; ++s) step_exact(v[(int64_t)s * st], s - 1, true, false);  // only an open run goes on
     return m;
 }
 
@@ -237,10 +259,11 @@ __host__ __device__ inline int dvdt_peaks_trace(const PeakArgs& a, int t) {
 
 // Blocks of 32 traces (lane = trace) and blockDim.y stretches of `stretch`
 // samples (even).  What bounds it: reading the traces once.  10,000 traces
-// of 3,168 samples (127 MB): 124 us with cold caches, 52 warp instructions
-// per 32 samples at 43 % issue activity.  One thread per trace (the form
-// this replaces) took 0.79 ms: two warps per SM, each walking 3,168 FP64
-// quotients one after another.
+// of 3,168 samples (127 MB): 89 us, 78 us where a trace's samples lie side by
+// side; comparing every difference in FP64 instead took 124 us (52 warp
+// instructions per 32 samples), one thread per trace 0.79 ms (two
+// warps per SM, each walking 3,168 FP64 quotients one after another).  Left:
+// 313 blocks of eight warps are two to three per SM, with 8 rows in flight.
 constexpr int kPeakList = 256;
 __global__ void __launch_bounds__(1024) k_dvdt_peaks(const PeakArgs a, int stretch, int row) {
     __shared__ int cnt[32][33];

@@ -102,3 +102,39 @@ def test_features_at_the_edges(ngpu_built, n, nt, layout):
         np.testing.assert_array_equal(got[:, 0], want[:, 0])
         # the statement's mean of an empty window is NaN, the kernel's 0 (a window past the trace's end)
         np.testing.assert_allclose(got, np.where(np.isnan(want), 0.0, want), rtol=2e-5, atol=2e-4)
+
+
+def _near_ties(rng, n):
+    """Rises past zero whose neighbouring slopes differ by less than a
+    float32 keeps, next to one that ends the peak or continues the rise."""
+    out = []
+    for k in range(n):
+        x2 = np.float32(rng.uniform(0.005, 0.02))
+        x3 = np.float32(48.0 + 2.0 * float(x2))
+        lead = [np.float32(-96.0)] * int(rng.integers(8, 24)) + [np.float32(-95.0 + rng.uniform(0, 1))]
+        out.append(np.array(lead + [-48.0, x2, x3, x3 + np.float32(48.5 if k % 2 else 40.0)] + [60.0] * 17,
+                            np.float32))
+    return out
+
+
+def test_slopes_that_round_alike(probe):
+    seen = set()
+    for x in _near_ties(np.random.default_rng(5), 400):
+        d = np.diff(x.astype(np.float64))
+        k = int(np.argmax(x == -48.0))
+        seen.add((np.sign(d[k + 1] - d[k]), bool(np.float32(d[k + 1]) == np.float32(d[k]))))
+        want = fpr.dvdt_peak_count(x, 0.1, 15.0, 1)
+        for stretch in (8, 16, 64):
+            assert probe.probe_stretches(x.ctypes.data, x.size, 1, 0.1, 15.0, 1, stretch) == want
+    assert {(1.0, True), (-1.0, True)} <= seen  # both orders, hidden by the rounding
+
+
+@pytest.mark.gpu
+def test_slopes_that_round_alike_on_the_gpu(ngpu_built):
+    import torch
+    from neurogpu_b200 import explore
+    rows = [x for x in _near_ties(np.random.default_rng(6), 400)]
+    v = np.stack([np.pad(x, (0, 64 - x.size), mode="edge") for x in rows])
+    want = [fpr.dvdt_peak_count(x, 0.1, 15.0, 1) for x in v]
+    got = explore.dvdt_peak_counts(torch.from_numpy(v).cuda(), distance=1).cpu().tolist()
+    assert got == want
