@@ -69,7 +69,14 @@ struct GemmArgs {
     const float* zin;        // [M][ldo]
     int* err;
     int kt_split;            // 64-wide K tiles per CTA; CTA z takes tiles [z kt_split, (z+1) kt_split)
+    int chained;             // (host) within a chain: launched during the kernel before; a split-K output is zero already
 };
+
+// Programmatic dependent launch: the next kernel of a chain may start (it
+// waits for this one's end before it touches memory), and this one waits for
+// the end of the kernel before.  Both do nothing outside a chain.
+__device__ __forceinline__ void dependent_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The tensor-core unit's tanh (tanh.approx.f32, one instruction; relative
 // error ~5e-4, below the bf16 rounding of the outputs it feeds).
@@ -390,6 +397,8 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm_bf16_tn(GemmArgs g) {
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = Sm.tmem;
+    dependent_launch();
+    dependent_wait();
 
     // this CTA's K tiles: [kt0, kt0 + KT) (the host gives every CTA at least one)
     const int kt0 = blockIdx.z * g.kt_split;
@@ -552,6 +561,8 @@ __global__ void __launch_bounds__(kTmaThreads) k_gemm_bf16_tma(const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = Sm.tmem;
+    dependent_launch();
+    dependent_wait();
 
     const int kt0 = blockIdx.z * g.kt_split;
     const int KT = min(g.kt_split, g.K / kGemmBK - kt0);
@@ -694,6 +705,8 @@ __global__ void __launch_bounds__(persist_threads(EPI), 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = Sm.tmem;
+    dependent_launch();
+    dependent_wait();
     bool ok = true;
 
     if (warp == 0) {

@@ -4,7 +4,11 @@
 // As elementwise torch operations these were ~90 launches of a training step
 // whose GEMMs take a tenth of a millisecond; each kernel here makes all that
 // its point of the step needs in one pass.  What bounds them is their launch:
-// a minibatch of 4,096 x 512 is a few megabytes.
+// a minibatch of 4,096 x 512 is a few megabytes.  So each kernel of a step is
+// launched while the one before it runs and waits for its end in
+// dependent_wait() (programmatic dependent launch), its first statement that
+// touches memory; a kernel ends only after its own wait, so waiting for the
+// one before is waiting for all.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -12,11 +16,27 @@
 
 namespace ngpu {
 
+// What the step's kernels add into, zeroed by its first kernel: one pass
+// instead of five memsets (1.4 us each and a gap).
+struct MlpZero {
+    float* p[4];
+    int n[4];
+    unsigned* done;
+};
+
 // xb[Mp][k_in] = bf16((X - mu) / sd), zero past M rows and n_in columns; xbt
 // its transpose (or nullptr).  mu, sd nullptr: X as it is.  One CTA per 32
-// rows, through shared memory so that both are written in rows.
+// rows, through shared memory so that both are written in rows.  zero: see
+// MlpZero.
 __global__ void __launch_bounds__(256) k_mlp_input(const float* X, int M, int n_in, const float* mu, const float* sd,
-                                                   int Mp, int k_in, __nv_bfloat16* xb, __nv_bfloat16* xbt) {
+                                                   int Mp, int k_in, __nv_bfloat16* xb, __nv_bfloat16* xbt,
+                                                   const MlpZero zero) {
+    dependent_launch();
+    const int threads = gridDim.x * gridDim.y * 256, id = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        for (int t = id; t < zero.n[k]; t += threads) zero.p[k][t] = 0.f;
+    if (zero.done && id == 0) *zero.done = 0;
     __shared__ __nv_bfloat16 tile[32][33];
     const int m0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int r = threadIdx.x >> 5; r < 32; r += 8) {
@@ -41,6 +61,7 @@ __global__ void __launch_bounds__(256) k_mlp_input(const float* X, int M, int n_
 // out[M][n_out] = y[.][n_out_p] * sd + mu (nullptr: y as it is)
 __global__ void __launch_bounds__(256) k_mlp_output(const float* y, int M, int n_out, int n_out_p, const float* mu,
                                                     const float* sd, float* out) {
+    dependent_wait();
     const size_t total = (size_t)M * n_out;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
         const size_t m = t / n_out;
@@ -77,16 +98,32 @@ __global__ void __launch_bounds__(256) k_mlp_loss(const MlpLossArgs a) {
     __shared__ bool last;
     const int m0 = blockIdx.x * kMlpLossRows;
     const float count = (float)((int64_t)a.M * a.n_out);
-    float sq = 0.f;
+    // a thread has eight rows of a column; their loads go out together (where
+    // each row's waited for the row before, the kernel took 14 us)
+    constexpr int kRows = kMlpLossRows / 4;
+    const int c = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+    const bool col = c < a.n_out;
+    float target[kRows], y[kRows], weight[kRows], sq = 0.f;
+    dependent_launch();
+    dependent_wait();
+    const float mu = col && a.mu ? a.mu[c] : 0.f, sd = col && a.mu ? a.sd[c] : 1.f;
 #pragma unroll
-    for (int t = threadIdx.x; t < kMlpLossRows * 64; t += 256) {
-        const int r = t >> 6, c = t & 63, m = m0 + r;
+    for (int k = 0; k < kRows; ++k) {
+        const int m = m0 + r0 + 4 * k;
+        const bool in = col && m < a.M;
+        target[k] = in ? a.Y[(size_t)m * a.n_out + c] : 0.f;
+        weight[k] = in && a.weight ? a.weight[m] : 1.f;
+        y[k] = in ? a.y[(size_t)m * a.n_out_p + c] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+        const int r = r0 + 4 * k, m = m0 + r;
         float dy = 0.f;
-        if (m < a.M && c < a.n_out) {
-            float target = a.Y[(size_t)m * a.n_out + c];
-            if (a.mu) target = __fdiv_rn(__fsub_rn(target, a.mu[c]), a.sd[c]);
-            float diff = __fsub_rn(a.y[(size_t)m * a.n_out_p + c], target);
-            if (a.weight) diff = __fmul_rn(diff, a.weight[m]);
+        if (col && m < a.M) {
+            float t = target[k];
+            if (a.mu) t = __fdiv_rn(__fsub_rn(t, mu), sd);
+            float diff = __fsub_rn(y[k], t);
+            if (a.weight) diff = __fmul_rn(diff, weight[k]);
             sq += diff * diff;
             dy = __fdiv_rn(2.0f * diff, count);
         }
@@ -97,17 +134,19 @@ __global__ void __launch_bounds__(256) k_mlp_loss(const MlpLossArgs a) {
     if ((threadIdx.x & 31) == 0) sq_s[threadIdx.x >> 5] = sq;
     __syncthreads();
     for (int t = threadIdx.x; t < a.n_out_p * kMlpLossRows; t += 256) {
-        const int c = t / kMlpLossRows, r = t % kMlpLossRows;
-        if (m0 + r < a.Mp) a.dybt[(size_t)c * a.Mp + m0 + r] = __float2bfloat16_rn(d_s[r][c]);
+        const int tc = t / kMlpLossRows, r = t % kMlpLossRows;
+        if (m0 + r < a.Mp) a.dybt[(size_t)tc * a.Mp + m0 + r] = __float2bfloat16_rn(d_s[r][tc]);
     }
     const int np = 1 + a.n_out_p;
-    for (int c = threadIdx.x; c < np; c += 256) {
+    if (threadIdx.x < np) {
         float s = 0.f;
-        if (c == 0)
+        if (threadIdx.x == 0) {
             for (int t = 0; t < 8; ++t) s += sq_s[t];
-        else
-            for (int r = 0; r < kMlpLossRows; ++r) s += d_s[r][c - 1];
-        a.part[(size_t)blockIdx.x * np + c] = s;
+        } else {
+#pragma unroll
+            for (int r = 0; r < kMlpLossRows; ++r) s += d_s[r][threadIdx.x - 1];
+        }
+        a.part[(size_t)blockIdx.x * np + threadIdx.x] = s;
     }
     __threadfence();
     __syncthreads();
@@ -117,17 +156,18 @@ __global__ void __launch_bounds__(256) k_mlp_loss(const MlpLossArgs a) {
     // four threads per sum, each every fourth block (np <= 65)
     __shared__ double sum_s[4][65];
     for (int t = threadIdx.x; t < 4 * np; t += 256) {
-        const int c = t % np, q = t / np;
+        const int k = t % np, q = t / np;
         double s = 0.0;
-#pragma unroll 8
-        for (unsigned b = q; b < gridDim.x; b += 4) s += (double)__ldcg(a.part + (size_t)b * np + c);
-        sum_s[q][c] = s;
+#pragma unroll 16
+        for (unsigned b = q; b < gridDim.x; b += 4) s += (double)__ldcg(a.part + (size_t)b * np + k);
+        sum_s[q][k] = s;
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < np; c += 256) {
-        const double s = (sum_s[0][c] + sum_s[1][c]) + (sum_s[2][c] + sum_s[3][c]);
-        if (c == 0) *a.loss = __fdiv_rn((float)s, count);
-        else a.gb[c - 1] = (float)s;
+    if (threadIdx.x < np) {
+        const int k = threadIdx.x;
+        const double s = (sum_s[0][k] + sum_s[1][k]) + (sum_s[2][k] + sum_s[3][k]);
+        if (k == 0) *a.loss = __fdiv_rn((float)s, count);
+        else a.gb[k - 1] = (float)s;
     }
 }
 
@@ -142,6 +182,7 @@ __global__ void __launch_bounds__(128) k_mlp_bias_grads(const MlpBiasArgs a) {
     const __nv_bfloat162* row =
         reinterpret_cast<const __nv_bfloat162*>(a.dzt[blockIdx.y] + (size_t)blockIdx.x * a.Mp);
     float s = 0.f;
+    dependent_wait();
     for (int t = threadIdx.x; t < a.Mp / 2; t += 128) {
         const float2 f = __bfloat1622float2(row[t]);
         s += f.x + f.y;
@@ -157,6 +198,8 @@ __global__ void __launch_bounds__(128) k_mlp_bias_grads(const MlpBiasArgs a) {
 __global__ void __launch_bounds__(256) k_mlp_transpose(const float* in, int rows, int cols, float* out) {
     __shared__ float tile[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32, x = threadIdx.x & 31;
+    dependent_launch();
+    dependent_wait();
     for (int k = threadIdx.x >> 5; k < 32; k += 8)
         if (r0 + k < rows && c0 + x < cols) tile[k][x] = in[(size_t)(r0 + k) * cols + c0 + x];
     __syncthreads();

@@ -2113,9 +2113,9 @@ static int feature_args(int32_t n_samples, double dt, double stim_on, double sti
 
 // Stretches of time a block's 32 traces are cut into (a warp each): enough
 // for about 16 warps per SM, at least 32 samples each.
-static int trace_stretches(int n_traces, int n_samples) {
+static int trace_stretches(int n_traces, int n_samples, int least) {
     const int blocks = (n_traces + 31) / 32;
-    int w = 8;
+    int w = least;
     while (w < 32 && blocks * w < 16 * kSmCount) w *= 2;
     while (w > 1 && n_samples < 32 * w) w /= 2;
     return w;
@@ -2130,10 +2130,14 @@ static int trace_rows(const float* v, int64_t stride_trace, int64_t stride_sampl
 
 static int launch_features(FeatureArgs a, cudaStream_t st) {
     if (a.n_traces < 1) return NGPU_OK;
-    const int w = trace_stretches(a.n_traces, a.n_samples);
+    // us with 8 / 16 / 32 stretches, 10,000 traces of 3,168 samples and 24,576
+    // of 2,000: traces side by side 168 / 135 / 126 and 181 / 135 / 174; a
+    // trace's samples side by side 103 / 165 / 184 (10,000)
+    const int row = trace_rows(a.v, a.stride_trace, a.stride_sample);
+    const int w = trace_stretches(a.n_traces, a.n_samples, a.stride_sample == 1 ? 8 : 16);
     const int smem = kFeatBytes * 32 * w;
     NGPU_CUDA(cudaFuncSetAttribute(k_trace_features, cudaFuncAttributeMaxDynamicSharedMemorySize, kFeatBytes * 32 * w));
-    k_trace_features<<<(a.n_traces + 31) / 32, dim3(32, w), smem, st>>>(a, trace_stretch(a.n_samples, w), trace_rows(a.v, a.stride_trace, a.stride_sample));
+    k_trace_features<<<(a.n_traces + 31) / 32, dim3(32, w), smem, st>>>(a, trace_stretch(a.n_samples, w), row);
     g_launches++;
     NGPU_CUDA(cudaGetLastError());
     return NGPU_OK;
@@ -2193,7 +2197,7 @@ static int launch_dvdt_peaks(PeakArgs a, int64_t scratch_bytes, cudaStream_t st)
         return fail(NGPU_E_INVALID, "dvdt peaks: scratch holds " + std::to_string(scratch_bytes) + " bytes, needs " +
                                         std::to_string(need));
     if (!a.v || !a.out || !a.pos) return fail(NGPU_E_INVALID, "dvdt peaks: null pointer");
-    const int w = trace_stretches(a.n_traces, a.n_samples);
+    const int w = trace_stretches(a.n_traces, a.n_samples, 8);
     k_dvdt_peaks<<<(a.n_traces + 31) / 32, dim3(32, w), sizeof(int32_t) * kPeakList * w, st>>>(
         a, trace_stretch(a.n_samples, w), trace_rows(a.v, a.stride_trace, a.stride_sample));
     g_launches++;
@@ -2703,6 +2707,29 @@ static bool gemm_use_persistent(int units) {
     return units > 2 * kSmCount;
 }
 
+// A launch that, in a chain, may begin during the kernel before it on the
+// stream (that kernel and this one order themselves by dependent_launch and
+// dependent_wait).  Hides the launches and the GEMMs' prologues: a training
+// step's 15 kernels up to the gradients (4,096 rows, width 512) take 114 us
+// from first to last, 163 with gaps of 1.7 us and five memsets between them; a
+// prediction of 24,576 rows 82 us, 92 without.
+template <typename... K, typename... A>
+static cudaError_t launch_chained(bool chained, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem,
+                                  cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    g_launches++;
+    return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+}
+
 template <int BN, int EPI>
 static cudaError_t launch_gemm_bn(GemmArgs g, cudaStream_t st) {
     if (gemm_use_tma(g, BN)) {
@@ -2717,29 +2744,25 @@ static cudaError_t launch_gemm_bn(GemmArgs g, cudaStream_t st) {
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) return e;
                 g.kt_split = per;
-                if (EPI == kEpiSplitAdd) {
+                if (EPI == kEpiSplitAdd && !g.chained) {
                     e = cudaMemsetAsync(g.out_f32, 0, sizeof(float) * ((size_t)(g.M - 1) * g.ldo + g.N), st);
                     if (e != cudaSuccess) return e;
                 }
                 const int units = n_mt * n_nt * splits;
-                k_gemm_bf16_tma_persistent<BN, EPI><<<std::min(units, kSmCount), persist_threads(EPI), smem, st>>>(
-                    ta, tb, g, units, n_mt, n_nt);
-                g_launches++;
-                return cudaGetLastError();
+                return launch_chained(g.chained, k_gemm_bf16_tma_persistent<BN, EPI>, std::min(units, kSmCount),
+                                      persist_threads(EPI), smem, st, ta, tb, g, units, n_mt, n_nt);
             }
             const size_t smem = gemm_tma_smem_bytes<BN>();
             cudaError_t e = cudaFuncSetAttribute(k_gemm_bf16_tma<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem);
             if (e != cudaSuccess) return e;
             g.kt_split = per;  // split-K: one CTA per SM, one wave
-            if (EPI == kEpiSplitAdd) {
+            if (EPI == kEpiSplitAdd && !g.chained) {
                 e = cudaMemsetAsync(g.out_f32, 0, sizeof(float) * ((size_t)(g.M - 1) * g.ldo + g.N), st);
                 if (e != cudaSuccess) return e;
             }
-            dim3 grid(n_mt, n_nt, splits);
-            k_gemm_bf16_tma<BN, EPI><<<grid, kTmaThreads, smem, st>>>(ta, tb, g);
-            g_launches++;
-            return cudaGetLastError();
+            return launch_chained(g.chained, k_gemm_bf16_tma<BN, EPI>, dim3(n_mt, n_nt, splits), kTmaThreads, smem, st,
+                                  ta, tb, g);
         }
     }
     const size_t smem = gemm_smem_bytes<BN>();
@@ -2747,14 +2770,12 @@ static cudaError_t launch_gemm_bn(GemmArgs g, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     int splits = 1;
     g.kt_split = gemm_k_split(g, BN, EPI, 2 * kSmCount, &splits);
-    if (EPI == kEpiSplitAdd) {  // the slices add into a zeroed output
+    if (EPI == kEpiSplitAdd && !g.chained) {  // the slices add into a zeroed output
         e = cudaMemsetAsync(g.out_f32, 0, sizeof(float) * ((size_t)(g.M - 1) * g.ldo + g.N), st);
         if (e != cudaSuccess) return e;
     }
     dim3 grid((g.M + kGemmBM - 1) / kGemmBM, (g.N + BN - 1) / BN, splits);
-    k_gemm_bf16_tn<BN, EPI><<<grid, kGemmThreads, smem, st>>>(g);
-    g_launches++;
-    return cudaGetLastError();
+    return launch_chained(g.chained, k_gemm_bf16_tn<BN, EPI>, grid, kGemmThreads, smem, st, g);
 }
 
 template <int EPI>
@@ -2770,7 +2791,8 @@ static cudaError_t launch_gemm_epi(GemmArgs g, int bn, cudaStream_t st) {
 // Checks and launch of one GEMM; epilogues up to `last` are known.
 static int gemm_checked(const void* A, const void* B, int32_t M, int32_t N, int32_t K, int32_t lda,
                         int32_t ldb, int32_t epilogue, int32_t bn, float* out_f32, void* out_bf16, void* out_bf16_t,
-                        int32_t ldo, int32_t ldt, const float* bias, const float* zin, void* cuda_stream, int last) {
+                        int32_t ldo, int32_t ldt, const float* bias, const float* zin, void* cuda_stream, int last,
+                        bool chained = false) {
     if (!A || !B) return fail(NGPU_E_INVALID, "gemm: null operand");
     if (M < 1 || N < 1 || K < kGemmBK || K % kGemmBK)
         return fail(NGPU_E_INVALID, "gemm: need M, N >= 1 and K a positive multiple of 64");
@@ -2791,7 +2813,7 @@ static int gemm_checked(const void* A, const void* B, int32_t M, int32_t N, int3
     cudaError_t e = cudaGetSymbolAddress((void**)&err, g_gemm_err);
     if (e != cudaSuccess) return fail(NGPU_E_CUDA, std::string("gemm: ") + cudaGetErrorString(e));
     GemmArgs g{(const __nv_bfloat16*)A, (const __nv_bfloat16*)B, M, N, K, lda, ldb, out_f32,
-               (__nv_bfloat16*)out_bf16, (__nv_bfloat16*)out_bf16_t, ldo, ldt, bias, zin, err, K / kGemmBK};
+               (__nv_bfloat16*)out_bf16, (__nv_bfloat16*)out_bf16_t, ldo, ldt, bias, zin, err, K / kGemmBK, chained};
     cudaStream_t st = (cudaStream_t)cuda_stream;
     switch (epilogue) {
         case kEpiStore: e = launch_gemm_epi<kEpiStore>(g, bn, st); break;
@@ -2905,20 +2927,22 @@ extern "C" int ngpu_mlp_predict(const float* X, int32_t M, int32_t n_in, const f
     const MlpPredictWs w(a, Mp, width, k_in, n_out_p);
     if (ws_bytes < a.used) return fail(NGPU_E_INVALID, "mlp_predict: workspace too small");
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    k_mlp_input<<<dim3(Mp / 32, k_in / 32), 256, 0, st>>>(X, M, n_in, x_mu, x_sd, Mp, k_in, w.xb, nullptr);
+    k_mlp_input<<<dim3(Mp / 32, k_in / 32), 256, 0, st>>>(X, M, n_in, x_mu, x_sd, Mp, k_in, w.xb, nullptr,
+                                                          MlpZero{});
+    g_launches++;
+    NGPU_CUDA(cudaGetLastError());
     const __nv_bfloat16* h = w.xb;
     for (int k = 0; k < 3; ++k) {
         __nv_bfloat16* o = k == 1 ? w.h1 : w.h0;
         const int kk = k == 0 ? k_in : width;
         NGPU_TRY(gemm_checked(h, wb[k], Mp, width, kk, kk, kk, kEpiGelu, bn, nullptr, o, nullptr, width, Mp, b[k],
-                              nullptr, st, kEpiGelu));
+                              nullptr, st, kEpiGelu, true));
         h = o;
     }
     NGPU_TRY(gemm_checked(h, wb[3], Mp, n_out_p, width, width, width, kEpiBias, 32, w.y, nullptr, nullptr, n_out_p, Mp,
-                          b[3], nullptr, st, kEpiGelu));
-    k_mlp_output<<<(unsigned)std::min<size_t>(((size_t)M * n_out + 255) / 256, 148 * 16), 256, 0, st>>>(w.y, M, n_out, n_out_p, y_mu, y_sd, out);
-    g_launches += 2;
-    NGPU_CUDA(cudaGetLastError());
+                          b[3], nullptr, st, kEpiGelu, true));
+    const unsigned blocks = (unsigned)std::min<size_t>(((size_t)M * n_out + 255) / 256, 148 * 16);
+    NGPU_CUDA(launch_chained(true, k_mlp_output, blocks, 256, 0, st, w.y, M, n_out, n_out_p, y_mu, y_sd, out));
     return NGPU_OK;
 }
 
@@ -2935,36 +2959,37 @@ extern "C" int ngpu_mlp_grads(const float* X, const float* Y, const float* weigh
     const MlpTrainWs w(a, Mp, width, k_in, n_out_p);
     if (ws_bytes < a.used) return fail(NGPU_E_INVALID, "mlp_grads: workspace too small");
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    k_mlp_input<<<dim3(Mp / 32, k_in / 32), 256, 0, st>>>(X, M, n_in, x_mu, x_sd, Mp, k_in, w.xb, w.ht[0]);
+    const MlpZero zero{{gw[0], gw[1], gw[2], w.g4t}, {width * k_in, width * width, width * width, width * n_out_p}, w.done};
+    k_mlp_input<<<dim3(Mp / 32, k_in / 32), 256, 0, st>>>(X, M, n_in, x_mu, x_sd, Mp, k_in, w.xb, w.ht[0], zero);
+    g_launches++;
+    NGPU_CUDA(cudaGetLastError());
     const __nv_bfloat16* h = w.xb;
     for (int k = 0; k < 3; ++k) {
         const int kk = k == 0 ? k_in : width;
         NGPU_TRY(gemm_checked(h, wb[k], Mp, width, kk, kk, kk, kEpiBiasGelu, bn, w.z[k], w.h[k], w.ht[k + 1], width, Mp,
-                              b[k], nullptr, st, kEpiGelu));
+                              b[k], nullptr, st, kEpiGelu, true));
         h = w.h[k];
     }
     NGPU_TRY(gemm_checked(h, wb[3], Mp, n_out_p, width, width, width, kEpiBias, 32, w.y, nullptr, nullptr, n_out_p, Mp,
-                          b[3], nullptr, st, kEpiGelu));
-    NGPU_CUDA(cudaMemsetAsync(w.done, 0, sizeof(unsigned), st));
+                          b[3], nullptr, st, kEpiGelu, true));
     const MlpLossArgs la{w.y, Y, y_mu, y_sd, weight, M, Mp, n_out, n_out_p, w.dyb, w.dybt, w.part, w.done, loss, gb[3]};
-    k_mlp_loss<<<(Mp + kMlpLossRows - 1) / kMlpLossRows, 256, 0, st>>>(la);
+    NGPU_CUDA(launch_chained(true, k_mlp_loss, (Mp + kMlpLossRows - 1) / kMlpLossRows, 256, 0, st, la));
     // output layer: dW^T[width][n_out_p] = H^T dY
     NGPU_TRY(gemm_checked(w.ht[3], w.dybt, width, n_out_p, Mp, Mp, Mp, kEpiSplitAdd, 32, w.g4t, nullptr, nullptr,
-                          n_out_p, width, nullptr, nullptr, st, kEpiGelu));
-    k_mlp_transpose<<<dim3((width + 31) / 32, n_out_p / 32), 256, 0, st>>>(w.g4t, width, n_out_p, gw[3]);
+                          n_out_p, width, nullptr, nullptr, st, kEpiGelu, true));
+    NGPU_CUDA(launch_chained(true, k_mlp_transpose, dim3((width + 31) / 32, n_out_p / 32), 256, 0, st, w.g4t, width,
+                             n_out_p, gw[3]));
     const __nv_bfloat16* dz = w.dyb;
     for (int k = 2; k >= 0; --k) {
         const int kd = k == 2 ? 64 : width, kin = k == 0 ? k_in : width;
         NGPU_TRY(gemm_checked(dz, wtb[k + 1], Mp, width, kd, kd, kd, kEpiGeluGrad, bn, nullptr, w.dzb[k], w.dzbt[k],
-                              width, Mp, nullptr, w.z[k], st, kEpiGelu));
+                              width, Mp, nullptr, w.z[k], st, kEpiGelu, true));
         NGPU_TRY(gemm_checked(w.dzbt[k], w.ht[k], width, kin, Mp, Mp, Mp, kEpiSplitAdd, kin == 64 ? 64 : 128,
-                              gw[k], nullptr, nullptr, kin, width, nullptr, nullptr, st, kEpiGelu));
+                              gw[k], nullptr, nullptr, kin, width, nullptr, nullptr, st, kEpiGelu, true));
         dz = w.dzb[k];
     }
     const MlpBiasArgs ba{{w.dzbt[0], w.dzbt[1], w.dzbt[2]}, {gb[0], gb[1], gb[2]}, Mp};
-    k_mlp_bias_grads<<<dim3(width, 3), 128, 0, st>>>(ba);
-    g_launches += 4;
-    NGPU_CUDA(cudaGetLastError());
+    NGPU_CUDA(launch_chained(true, k_mlp_bias_grads, dim3(width, 3), 128, 0, st, ba));
     return NGPU_OK;
 }
 

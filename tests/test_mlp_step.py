@@ -111,3 +111,43 @@ def test_gradients_and_step(ngpu_built, rows, width, n_out, weighted):
         assert torch.equal(net.Wb[k], w)
         wt_ = torch.nn.functional.pad(w.t(), (0, 64 - net.n_out_p)) if k == 3 else w.t()
         assert torch.equal(net.Wtb[k], wt_)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,width", [(100, 64), (4096, 512), (20000, 512)])
+def test_chained_kernels_keep_their_order(ngpu_built, rows, width):
+    """Calls back to back, whose workspaces are the same memory, and replayed
+    from a CUDA graph give what each call gives alone (split sums of the
+    weight gradients add in any order: 4,096 terms of FP32)."""
+    import torch
+    net = _net(15, 20, width, True)
+    data = [_data(rows, 15, 20, 50 + k) for k in range(6)]
+
+    def step(X, Y):
+        loss, gW, gb = net.loss_and_grads(X, Y)
+        return [net.predict(X), loss, *gb, *gW]
+
+    alone = []
+    for X, Y in data:
+        alone.append([t.clone() for t in step(X, Y)])
+        torch.cuda.synchronize()
+
+    def same(got, want):
+        for k, (g, w) in enumerate(zip(got, want)):
+            if k < 6:
+                assert torch.equal(g, w), k
+            else:
+                assert float((g - w).norm()) <= 1e-5 * float(w.norm()), k
+
+    for got, want in zip([step(X, Y) for X, Y in data], alone):
+        same(got, want)
+    X, Y = data[0][0].clone(), data[0][1].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step(X, Y)
+    for (x, y), want in zip(data, alone):
+        X.copy_(x)
+        Y.copy_(y)
+        graph.replay()
+        torch.cuda.synchronize()
+        same(out, want)
