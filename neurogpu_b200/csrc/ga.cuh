@@ -266,29 +266,70 @@ __global__ void k_ga_take(const uint32_t* sorted_idx, int mu, int32_t* out) {
 constexpr int kGaSmallMax = 16384;
 constexpr int kGaDomThreads = 256;
 
-// Sorts (key, index) pairs in shared memory, ascending by key, then index; n2
-// a power of two >= 64.  A thread takes pairs; while a pair's distance is
-// within a warp's 64 entries a warp barrier orders the stages.
-__device__ __forceinline__ void ga_bitonic(uint64_t* key, uint16_t* idx, uint32_t n2) {
-    for (uint32_t k = 2; k <= n2; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t t = threadIdx.x; t < n2 / 2; t += blockDim.x) {
-                const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), l = i | j;
-                const uint64_t x = key[i], y = key[l];
-                const uint16_t xi = idx[i], yi = idx[l];
-                const bool less = (y < x) | ((y == x) & (yi < xi));  // entry l belongs before entry i
-                if (less == ((i & k) == 0)) {
-                    key[i] = y;
-                    key[l] = x;
-                    idx[i] = yi;
-                    idx[l] = xi;
-                }
-            }
-            if (j > 32 || (j == 1 && k >= 64)) __syncthreads();
-            else __syncwarp();
+// Sorts a CTA's (key, index) pairs, ascending by key, then index: eight per
+// thread in registers (n2 = 8 x threads, a power of two >= 256), entry e at
+// thread e / 8.  A bitonic network, whose stages of distance 1 to 4 are
+// within a thread, 8 to 128 within a warp (shuffles), and only those of 256
+// and more go through shared memory: 6 of the 66 stages of 2,048 entries.
+// With every stage there (a thread a pair), it was bound by its wavefronts:
+// 60 x 5 tiles of 2,048 took 61 us, now 43 (compares, of 64-bit keys).
+constexpr int kGaPer = 8;
+__device__ __forceinline__ bool ga_less(uint64_t x, uint32_t xi, uint64_t y, uint32_t yi) {
+    return (x < y) | ((x == y) & (xi < yi));
+}
+template <int J>
+__device__ __forceinline__ void ga_stage_thread(uint64_t (&x)[kGaPer], uint32_t (&id)[kGaPer], uint32_t k) {
+#pragma unroll
+    for (int u = 0; u < kGaPer; ++u) {
+        if (u & J) continue;
+        const bool up = ((threadIdx.x * kGaPer + u) & k) == 0;
+        if (ga_less(x[u | J], id[u | J], x[u], id[u]) == up) {
+            const uint64_t t = x[u];
+            x[u] = x[u | J];
+            x[u | J] = t;
+            const uint32_t ti = id[u];
+            id[u] = id[u | J];
+            id[u | J] = ti;
         }
     }
-    __syncthreads();
+}
+__device__ __forceinline__ void ga_bitonic(uint64_t (&x)[kGaPer], uint32_t (&id)[kGaPer], uint64_t* key_s,
+                                           uint16_t* idx_s, uint32_t n2) {
+    const uint32_t T = n2 / kGaPer, tid = threadIdx.x;
+    for (uint32_t k = 2; k <= n2; k <<= 1) {
+        for (uint32_t j = k >> 1; j >= kGaPer; j >>= 1) {
+            const uint32_t d = j / kGaPer;  // the partner thread's distance
+            const bool least = ((tid & d) == 0) == ((tid * kGaPer & k) == 0);
+            if (d >= 32) {
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < kGaPer; ++u) {
+                    key_s[u * T + tid] = x[u];
+                    idx_s[u * T + tid] = (uint16_t)id[u];
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int u = 0; u < kGaPer; ++u) {
+                uint64_t y;
+                uint32_t yi;
+                if (d >= 32) {
+                    y = key_s[u * T + (tid ^ d)];
+                    yi = idx_s[u * T + (tid ^ d)];
+                } else {
+                    y = __shfl_xor_sync(0xFFFFFFFFu, x[u], d);
+                    yi = __shfl_xor_sync(0xFFFFFFFFu, id[u], d);
+                }
+                if (ga_less(y, yi, x[u], id[u]) == least) {
+                    x[u] = y;
+                    id[u] = yi;
+                }
+            }
+        }
+        if (k >= 8) ga_stage_thread<4>(x, id, k);
+        if (k >= 4) ga_stage_thread<2>(x, id, k);
+        ga_stage_thread<1>(x, id, k);
+    }
 }
 
 // An objective's value as a key (NaN as +inf, the worst).
@@ -299,14 +340,14 @@ __device__ __forceinline__ uint64_t ga_obj_key(double x) { return ga_order_key(x
 // counted by a binary search in every tile (k_ga_places).  Keys: the
 // objective's value (FRONTS false), or the front and the place in the
 // objective's order, which makes the order within each front.  One CTA per
-// objective sorting all of it took 271 us for 60 x 10,000 (36 with both steps).
+// objective sorting all of it took 271 us for 60 x 10,000; the two steps take 43 + 36.
 constexpr int kGaTile = 2048;
 struct GaOrderArgs {
     const double* obj;       // [n][m]
     const int32_t* rank;     // [n] fronts (FRONTS)
     const int32_t* n_fronts; // (FRONTS)
     int n, m;
-    uint32_t tile;           // entries per tile, a power of two >= 64
+    uint32_t tile;           // entries per tile, a power of two >= 256
     uint64_t* key;           // [m][tiles * tile] sorted tiles
     uint16_t* idx;
     uint16_t* order;         // [m][n] individuals in the objective's order
@@ -314,32 +355,35 @@ struct GaOrderArgs {
     uint16_t* in_fronts;     // [m][n] individuals by front, then in the objective's order (FRONTS)
 };
 template <bool FRONTS>
-__global__ void __launch_bounds__(kGaTile / 2) k_ga_tiles(const GaOrderArgs a) {
+__global__ void __launch_bounds__(kGaTile / kGaPer) k_ga_tiles(const GaOrderArgs a) {
     __shared__ uint64_t key[kGaTile];
     __shared__ uint16_t idx[kGaTile];
     const int k = blockIdx.y;
-    const size_t base = ((size_t)k * gridDim.x + blockIdx.x) * a.tile;
-    for (uint32_t t = threadIdx.x; t < a.tile; t += blockDim.x) {
-        const int p = blockIdx.x * (int)a.tile + (int)t;
-        uint64_t x = ~0ull;
-        int i = p;
+    const uint32_t T = a.tile / kGaPer;
+    uint64_t x[kGaPer];
+    uint32_t id[kGaPer];
+#pragma unroll
+    for (int u = 0; u < kGaPer; ++u) {
+        const int p = blockIdx.x * (int)a.tile + (int)(u * T + threadIdx.x);
+        x[u] = ~0ull;
+        id[u] = p;
         if (p < a.n) {
             if constexpr (FRONTS) {
-                i = a.order[(size_t)k * a.n + p];
-                x = ((uint64_t)a.rank[i] << 14) | (uint32_t)p;
+                id[u] = a.order[(size_t)k * a.n + p];
+                x[u] = ((uint64_t)a.rank[id[u]] << 14) | (uint32_t)p;
             } else {
-                x = ga_obj_key(a.obj[(size_t)i * a.m + k]);
+                x[u] = ga_obj_key(a.obj[(size_t)p * a.m + k]);
             }
         }
-        key[t] = x;
-        idx[t] = (uint16_t)i;
     }
-    __syncthreads();
-    if (!FRONTS || *a.n_fronts > 1)  // (a single front is in order already)
-        ga_bitonic(key, idx, a.tile);
-    for (uint32_t t = threadIdx.x; t < a.tile; t += blockDim.x) {
-        a.key[base + t] = key[t];
-        a.idx[base + t] = idx[t];
+    const bool sort = !FRONTS || *a.n_fronts > 1;  // (a single front is in order already)
+    if (sort) ga_bitonic(x, id, key, idx, a.tile);
+    const size_t base = ((size_t)k * gridDim.x + blockIdx.x) * a.tile;
+#pragma unroll
+    for (int u = 0; u < kGaPer; ++u) {
+        const uint32_t t = sort ? threadIdx.x * kGaPer + u : u * T + threadIdx.x;
+        a.key[base + t] = x[u];
+        a.idx[base + t] = (uint16_t)id[u];
     }
 }
 

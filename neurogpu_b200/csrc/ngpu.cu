@@ -3152,7 +3152,7 @@ static int select_nsga2_small(const double* obj, int n, int m, int mu, int32_t* 
     int rc = NGPU_OK;
     StreamScratch ws(st);
     const int W = (n + 31) / 32, q = (m + 1) / 2, b = (n + 255) / 256;
-    const uint32_t tile = std::min<uint32_t>(kGaTile, std::max<uint32_t>(64, pow2_at_least(n)));
+    const uint32_t tile = std::min<uint32_t>(kGaTile, std::max<uint32_t>(32 * kGaPer, pow2_at_least(n)));
     const int tiles = (int)((n + tile - 1) / tile);
     const dim3 pairs(b, (n + kGaCount - 1) / kGaCount);
     uint16_t* order = ws.get<uint16_t>((size_t)m * n, &rc);
@@ -3172,7 +3172,7 @@ static int select_nsga2_small(const double* obj, int n, int m, int mu, int32_t* 
     uint64_t* key = ws.get<uint64_t>(n, &rc);
     if (rc != NGPU_OK) return rc;
     const GaOrderArgs oa{obj, rank, n_fronts, n, m, tile, tile_key, tile_idx, order, (uint16_t*)rank2, in_fronts};
-    k_ga_tiles<false><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
+    k_ga_tiles<false><<<dim3(tiles, m), tile / kGaPer, 0, st>>>(oa);
     k_ga_places<false><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
     k_ga_rank_sums<<<b, 256, 0, st>>>(rank2, n, q, sum, seat);
     k_ga_seats_sum<<<pairs, 256, 0, st>>>(sum, n, seat);
@@ -3190,7 +3190,7 @@ static int select_nsga2_small(const double* obj, int n, int m, int mu, int32_t* 
         void* args[] = {&fa};
         NGPU_CUDA(cudaLaunchCooperativeKernel((const void*)k_ga_fronts_count, dim3(blocks), dim3(kGaDomThreads), args, 0, st));
     }
-    k_ga_tiles<true><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
+    k_ga_tiles<true><<<dim3(tiles, m), tile / kGaPer, 0, st>>>(oa);
     k_ga_places<true><<<dim3(tiles, m), tile / 2, 0, st>>>(oa);
     k_ga_crowd_small<<<dim3(b, m), 256, 0, st>>>(GaCrowdSmallArgs{obj, in_fronts, rank, start, n, m, contrib});
     k_ga_crowd_seats<<<b, 256, 0, st>>>(contrib, rank, start, n, m, crowd, key, seat);
