@@ -20,7 +20,7 @@ namespace ngpu {
 // instead of five memsets (1.4 us each and a gap).
 struct MlpZero {
     float* p[4];
-    int n[4];
+    int64_t n[4];
     unsigned* done;
 };
 
@@ -32,10 +32,11 @@ __global__ void __launch_bounds__(256) k_mlp_input(const float* X, int M, int n_
                                                    int Mp, int k_in, __nv_bfloat16* xb, __nv_bfloat16* xbt,
                                                    const MlpZero zero) {
     dependent_launch();
-    const int threads = gridDim.x * gridDim.y * 256, id = (blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x;
+    const int64_t threads = (int64_t)gridDim.x * gridDim.y * 256;
+    const int64_t id = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 256 + threadIdx.x;
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        for (int t = id; t < zero.n[k]; t += threads) zero.p[k][t] = 0.f;
+        for (int64_t t = id; t < zero.n[k]; t += threads) zero.p[k][t] = 0.f;
     if (zero.done && id == 0) *zero.done = 0;
     __shared__ __nv_bfloat16 tile[32][33];
     const int m0 = blockIdx.x * 32, c0 = blockIdx.y * 32;

@@ -2130,9 +2130,11 @@ static int trace_rows(const float* v, int64_t stride_trace, int64_t stride_sampl
 
 static int launch_features(FeatureArgs a, cudaStream_t st) {
     if (a.n_traces < 1) return NGPU_OK;
-    // us with 8 / 16 / 32 stretches, 10,000 traces of 3,168 samples and 24,576
-    // of 2,000: traces side by side 168 / 135 / 126 and 181 / 135 / 174; a
-    // trace's samples side by side 103 / 165 / 184 (10,000)
+    // The blocks' shared memory (7 KB a warp) lets few of them share an SM, so
+    // their number decides how evenly SMs fill.  us with 8 / 16 / 32
+    // stretches, 10,000 traces of 3,168 samples and 24,576 of 2,000: traces
+    // side by side 168 / 135 / 126 and 181 / 135 / 174; a trace's samples side
+    // by side 103 / 165 / 184 (10,000), which reads through L1.
     const int row = trace_rows(a.v, a.stride_trace, a.stride_sample);
     const int w = trace_stretches(a.n_traces, a.n_samples, a.stride_sample == 1 ? 8 : 16);
     const int smem = kFeatBytes * 32 * w;
@@ -2959,7 +2961,8 @@ extern "C" int ngpu_mlp_grads(const float* X, const float* Y, const float* weigh
     const MlpTrainWs w(a, Mp, width, k_in, n_out_p);
     if (ws_bytes < a.used) return fail(NGPU_E_INVALID, "mlp_grads: workspace too small");
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    const MlpZero zero{{gw[0], gw[1], gw[2], w.g4t}, {width * k_in, width * width, width * width, width * n_out_p}, w.done};
+    const int64_t wide = width;
+    const MlpZero zero{{gw[0], gw[1], gw[2], w.g4t}, {wide * k_in, wide * width, wide * width, wide * n_out_p}, w.done};
     k_mlp_input<<<dim3(Mp / 32, k_in / 32), 256, 0, st>>>(X, M, n_in, x_mu, x_sd, Mp, k_in, w.xb, w.ht[0], zero);
     g_launches++;
     NGPU_CUDA(cudaGetLastError());
