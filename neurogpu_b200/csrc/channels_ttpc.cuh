@@ -278,7 +278,7 @@ NGPU_HD void ttpc_node(MK mk, R v, R dt, R* __restrict__ st, const float* __rest
     if (mk & TTPC::kCaDyn) {  // AllModels.cu:222-225 (init), :313-317 (cnexp, previous step's ica)
         if (INIT) cai = (R)kDefCai;
         else {
-            R cinf = (R)(-10000.0 / (2.0 * kFaraday)) * M::dv(ica * gamma, depth) * decay + mincai;
+            R cinf = ((R)(-10000.0 / (2.0 * kFaraday)) * M::dv(ica * gamma, depth) + M::dv(mincai, decay)) * decay;
             cai = cnexp_rate(cai, cinf, M::rc(decay), dt);
         }
     }
@@ -326,7 +326,7 @@ NGPU_HD void ttpc_node(MK mk, R v, R dt, R* __restrict__ st, const float* __rest
     // Ca currents with eca from the updated cai (AllModels.cu:382-407)
     ica = 0;
     if (mk & (TTPC::kCaHVA | TTPC::kCaLVA)) {
-        R eca = (R)(ktf_of(TTPC::kCelsius) / 2) * ((R)kLogCao - M::lg(cai));
+        R eca = (R)(ktf_of(TTPC::kCelsius) / 2) * M::lg(M::dv((R)kDefCao, cai));
         R gca = g_hva * hva_m * hva_m * hva_h + g_lva * lva_m * lva_m * lva_h;
         ica = gca * (v - eca);
         Itot += ica; Gtot += gca;
