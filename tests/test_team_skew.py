@@ -16,8 +16,8 @@ import pytest
 ROOT = Path(__file__).resolve().parents[1]
 HEADERS = ["ngpu_math.cuh", "param_fold.cuh", "node_classes.cuh", "channels_ttpc.cuh", "channels_mainen.cuh",
            "sim_kernels.cuh"]
-RANK = "        rank = cluster_rank();\n"
-DELAY = "        if (rank == t0 % A.team) for (int k = 0; k < 250; ++k) __nanosleep(1000);\n"
+START = "    Group<R> G = group_of(A, g);\n    const int w = threadIdx.x >> 5;\n    const NodeRec<R>* nr = stage_nodes(A, smem);\n"
+DELAY = "    if (TEAM && cluster_rank() == t0 % A.team) for (int k = 0; k < 250; ++k) __nanosleep(1000);\n"
 
 RUN = """
 import sys
@@ -57,9 +57,9 @@ def _kernel(tmp, unit, name, delay):
     for h in HEADERS:
         shutil.copy(ROOT / "neurogpu_b200" / "csrc" / h, inc / h)
     text = (inc / "sim_kernels.cuh").read_text()
-    assert text.count(RANK) == 1
+    assert text.count(START) == 1
     if delay:
-        (inc / "sim_kernels.cuh").write_text(text.replace(RANK, RANK + DELAY))
+        (inc / "sim_kernels.cuh").write_text(text.replace(START, DELAY + START))
     cubin = inc / "unit.cubin"
     subprocess.run(["nvcc", "-cubin", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-I", str(inc),
                     str(unit), "-o", str(cubin)], check=True, capture_output=True)
