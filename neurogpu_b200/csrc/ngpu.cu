@@ -2138,7 +2138,9 @@ static int launch_features(FeatureArgs a, cudaStream_t st) {
     const int row = trace_rows(a.v, a.stride_trace, a.stride_sample);
     const int w = trace_stretches(a.n_traces, a.n_samples, a.stride_sample == 1 ? 8 : 16);
     const int smem = kFeatBytes * 32 * w;
-    NGPU_CUDA(cudaFuncSetAttribute(k_trace_features, cudaFuncAttributeMaxDynamicSharedMemorySize, kFeatBytes * 32 * w));
+    // the limit belongs to the kernel, not to this launch: always the largest
+    // (32 stretches), so that calls of several threads set the same
+    NGPU_CUDA(cudaFuncSetAttribute(k_trace_features, cudaFuncAttributeMaxDynamicSharedMemorySize, kFeatBytes * 32 * 32));
     k_trace_features<<<(a.n_traces + 31) / 32, dim3(32, w), smem, st>>>(a, trace_stretch(a.n_samples, w), row);
     g_launches++;
     NGPU_CUDA(cudaGetLastError());
