@@ -527,7 +527,7 @@ struct ngpu_sim {
     ngpu_batch* batch = nullptr;  // the batch whose kernels this simulation's records follow
     int s2_stage = 0;             // skeleton solved from shared memory (see sim_kernels.cuh)
     int items_per_warp = 3;       // work items per warp in the tree split
-    bool items_chosen = false;    // ... given by the caller
+    bool items_chosen = false;    // ... given by the caller or the environment
     ngpu_jit::Folds folds;        // parameters the runtime-specialised kernel compiles in
     uint2* d_prange = nullptr;    // [ptab_rows] bit-pattern range of each parameter row
     unsigned long long* d_phash = nullptr;  // [ptab_rows] hash of each parameter row
@@ -1179,7 +1179,10 @@ static void sim_split_lanes(ngpu_sim* s) {
         skeleton_tables(s->part);
         s->s2_stage = f8 ? choose_s2_stage<double>(m->n, s->part, s->n_warps, s->ctas)
                          : choose_s2_stage<float>(m->n, s->part, s->n_warps, s->ctas);
-        if (s->s2_stage || s->items_chosen || s->n_warps < 2) return;
+        if (s->s2_stage || s->items_chosen || s->n_warps < 2) {
+            s->items_per_warp = k;  // (what ngpu_sim_layout tells)
+            return;
+        }
     }
     s->part = make_partition(m, s->n_warps, s->items_per_warp);
     skeleton_tables(s->part);
@@ -1299,9 +1302,14 @@ int ngpu_sim_create_layout(ngpu_model* m, int32_t n_sets, int32_t n_stim, int32_
     W = std::min(W, m->n);
     s->n_warps = W;
     s->items_per_warp = default_items(W);
-    if (const char* ev = getenv("NGPU_ITEMS_PER_WARP")) s->items_per_warp = std::max(1, std::min(8, atoi(ev)));
-    if (items_per_warp > 0) s->items_per_warp = items_per_warp;
-    s->items_chosen = items_per_warp > 0;
+    if (const char* ev = getenv("NGPU_ITEMS_PER_WARP")) {
+        s->items_per_warp = std::max(1, std::min(8, atoi(ev)));
+        s->items_chosen = true;
+    }
+    if (items_per_warp > 0) {
+        s->items_per_warp = items_per_warp;
+        s->items_chosen = true;
+    }
     if (ti) {
         // one warp per instance: the tree split into ti_items items for the
         // warp's lanes; CTAs of ti_warps instances, enough CTAs for every SM
