@@ -491,9 +491,10 @@ struct ngpu_sim {
     void* d_sepv = nullptr;
     int n_warps = 1;
     bool warps_chosen = false;    // ... given by the caller
-    bool no_team = false;         // while a batch splits it
     int ctas = 3;                 // CTAs per SM the batch is laid out for (kernels above 8 warps: compiled for)
     int team = 0;                 // CTAs (of n_warps warps) per group, one cluster; 0: one CTA per group
+    int split_warps = 0;          // at the next initialisation: split again, for CTAs of this many warps
+    int split_ctas = 0;           // ... and CTAs per SM (0 warps: stay)
     int* d_skel = nullptr;        // the staged skeleton's tables (part.skel)
     int* d_team_items = nullptr;
     Partition part;
@@ -1155,11 +1156,11 @@ static void host_copy_parallel(void* dst, const void* src, size_t bytes) {
 
 // The tree split of a lane-instance simulation for its n_warps, items_per_warp
 // and batch size.
-static void sim_split_lanes(ngpu_sim* s) {
+static void sim_split_lanes(ngpu_sim* s, bool teams = true) {
     const ngpu_model* m = s->m;
     const bool f8 = s->precision == NGPU_FP64;
     s->team = 0;
-    int team = s->n_warps > kMaxWarps && s->ctas == 1 && !s->no_team ? team_size(s->n_groups, m->n) : 0;
+    int team = s->n_warps > kMaxWarps && s->ctas == 1 && teams ? team_size(s->n_groups, m->n) : 0;
     if (const char* ev = getenv("NGPU_TEAM")) team = std::min(team, atoi(ev));
     for (; team > 1; --team) {
         s->part = make_partition(m, s->n_warps * team, s->items_per_warp);
@@ -1225,6 +1226,67 @@ static int sim_upload_split(ngpu_sim* s) {
         NGPU_CUDA(cudaMemcpy(s->d_team_items, ti.data(), sizeof(int) * ti.size(), cudaMemcpyHostToDevice));
     }
     return NGPU_OK;
+}
+
+// CTAs of `warps` warps (at most; one per group), `ctas` per SM, for a
+// simulation that is to be initialised: its tree is split for them.  After a
+// failed allocation the next initialisation splits first.
+static int sim_split_again(ngpu_sim* s, int warps, int ctas) {
+    s->initialized = false;
+    s->split_warps = warps;
+    s->split_ctas = ctas;
+    s->n_warps = warps;
+    s->ctas = ctas;
+    if (!s->items_chosen) s->items_per_warp = default_items(warps);
+    sim_split_lanes(s, false);
+    const int rc = sim_upload_split(s);
+    if (rc == NGPU_OK) s->split_warps = 0;
+    return rc;
+}
+
+extern "C++" {
+// The same for a simulation that is under way, whose numbers are laid out for
+// its split: it keeps the split (any number of warps can share the items),
+// as one CTA per group.
+template <typename R>
+static int sim_narrow(ngpu_sim* s, int warps, int ctas) {
+    if (s->team) {
+        const size_t G = (size_t)s->n_groups, L = kLanes, nj = (size_t)s->part.n_jslots, ns = s->part.seps.size();
+        int rc = NGPU_OK;
+        double* jacc = (double*)dmalloc(G * 2 * nj * L * sizeof(double), &rc);
+        if (!jacc) return rc;
+        R* sepv = (R*)dmalloc(G * 4 * ns * L * sizeof(R), &rc);
+        cudaError_t e = cudaSuccess;
+        if (sepv) {
+            e = cudaDeviceSynchronize();  // (its steps may be on any stream)
+            if (e == cudaSuccess) {
+                k_leave_team<R><<<s->n_groups, 256>>>(make_args<R>(s), jacc, sepv);
+                g_launches++;
+                e = cudaGetLastError();
+            }
+            if (e == cudaSuccess) e = cudaDeviceSynchronize();
+        }
+        if (!sepv || e != cudaSuccess) {
+            cudaFree(jacc);
+            cudaFree(sepv);
+            return sepv ? fail(NGPU_E_CUDA, std::string("split: ") + cudaGetErrorString(e)) : rc;
+        }
+        cudaFree(s->d_jacc);
+        cudaFree(s->d_sepv);
+        cudaFree(s->d_team_items);
+        s->d_jacc = jacc;
+        s->d_sepv = sepv;
+        s->d_team_items = nullptr;
+        s->team = 0;
+    }
+    s->n_warps = std::min(s->n_warps, warps);
+    s->ctas = ctas;
+    s->s2_stage = choose_s2_stage<R>(s->m->n, s->part, s->n_warps, ctas);
+    return NGPU_OK;
+}
+static int sim_narrow(ngpu_sim* s, int warps, int ctas) {
+    return s->precision == NGPU_FP64 ? sim_narrow<double>(s, warps, ctas) : sim_narrow<float>(s, warps, ctas);
+}
 }
 
 int ngpu_sim_create(ngpu_model* m, int32_t n_sets, int32_t n_stim, int32_t precision,
@@ -1464,6 +1526,7 @@ static int sim_share_param_blocks(ngpu_sim* s, std::vector<int32_t>* canon_out) 
 extern "C++" {  // defined with the batch, outside this C-linkage block
 static const ngpu_jit::Folds& batch_folds(const ngpu_batch* b);
 static int batch_refold(ngpu_batch* b);
+static void batch_size_smem(ngpu_batch* b);
 }
 
 static int sim_find_folds(ngpu_sim* s) {
@@ -1644,6 +1707,11 @@ static int sim_prepare_init(ngpu_sim* s, float v_init, cudaStream_t st) {
     if (!s->has_params) return fail(NGPU_E_STATE, "set_params must precede init");
     if (!s->has_stim) return fail(NGPU_E_STATE, "set_stimulus must precede init");
     if (!std::isfinite(v_init)) return fail(NGPU_E_INVALID, "v_init must be finite");
+    if (s->split_warps) {  // the split its batch asked for, now that its state may go
+        const int rc = sim_split_again(s, s->split_warps, s->split_ctas);
+        if (rc != NGPU_OK) return rc;
+        if (s->batch) batch_size_smem(s->batch);
+    }
     const int rc = sim_upload_nodes(s);
     if (rc != NGPU_OK) return rc;
     s->n_samples = (s->nt + s->rec_every - 1) / s->rec_every;
@@ -1874,6 +1942,14 @@ static void batch_drop_graph(ngpu_batch* b) {
     b->graph_key.clear();
 }
 
+// Dynamic shared memory of the batch's CTAs: what the largest member needs.
+static void batch_size_smem(ngpu_batch* b) {
+    b->smem = 0;
+    for (ngpu_sim* s : b->sims)
+        b->smem = std::max(b->smem, b->precision == NGPU_FP64 ? lane_smem<double>(s->m->n, s->part, s->s2_stage)
+                                                             : lane_smem<float>(s->m->n, s->part, s->s2_stage));
+}
+
 // One specialised kernel over every member's masks, with the parameters all
 // members share compiled in.
 static int batch_select_kernels(ngpu_batch* b) {
@@ -1917,8 +1993,9 @@ int ngpu_batch_create(ngpu_sim* const* sims, int32_t n, ngpu_batch** out) {
     }
     // one launch, one CTA shape: members whose warps the library chose (or
     // wider ones than 8) are split again for the CTAs per SM that the whole
-    // batch is laid out for, and must be initialised again (through the batch);
-    // a batch of at most one group per SM keeps CTAs of up to 8
+    // batch is laid out for; one that is under way keeps its split until it
+    // is initialised again.  A batch of at most one group per SM keeps CTAs of
+    // up to 8 warps
     const bool f8 = sims[0]->precision == NGPU_FP64;
     size_t plain = 0;
     int groups = 0;
@@ -1928,34 +2005,31 @@ int ngpu_batch_create(ngpu_sim* const* sims, int32_t n, ngpu_batch** out) {
     }
     const bool wide = groups > kSmCount && ngpu_jit::enabled() && ngpu_jit::nvrtc().ok;
     const int ctas = wide ? resident_ctas(plain, groups) : std::min(3, ctas_by_smem(plain));
+    int width = 1;
     for (int k = 0; k < n; ++k) {
         ngpu_sim* s = sims[k];
-        if (s->warps_chosen && s->n_warps <= kMaxWarps) continue;
+        if (s->warps_chosen && s->n_warps <= kMaxWarps) {
+            width = std::max(width, s->n_warps);
+            continue;
+        }
         const int W = default_warps(s->m->n, wide && !s->warps_chosen ? resident_warps(ctas) : kMaxWarps);
+        width = std::max(width, W);
         if (W == s->n_warps && !s->team && s->ctas == ctas) continue;
-        s->n_warps = W;
-        s->ctas = ctas;
-        if (!s->items_chosen) s->items_per_warp = default_items(W);
-        s->no_team = true;
-        sim_split_lanes(s);
-        s->no_team = false;
-        const int rc = sim_upload_split(s);
+        if (s->initialized) {
+            s->split_warps = W;
+            s->split_ctas = ctas;
+        }
+        const int rc = s->initialized ? sim_narrow(s, W, ctas) : sim_split_again(s, W, ctas);
         if (rc != NGPU_OK) return rc;
-        s->initialized = false;
     }
     ngpu_batch* b = new (std::nothrow) ngpu_batch();
     if (!b) return fail(NGPU_E_NOMEM, "host allocation failed");
     b->sims.assign(sims, sims + n);
     b->precision = sims[0]->precision;
     b->mechset = sims[0]->m->mechset;
-    int W = 1;
-    for (ngpu_sim* s : b->sims) {
-        W = std::max(W, s->n_warps);
-        b->total_ctas += s->n_groups;
-        b->smem = std::max(b->smem, b->precision == NGPU_FP64 ? lane_smem<double>(s->m->n, s->part, s->s2_stage)
-                                                             : lane_smem<float>(s->m->n, s->part, s->s2_stage));
-    }
-    b->threads = kLanes * W;
+    for (ngpu_sim* s : b->sims) b->total_ctas += s->n_groups;
+    batch_size_smem(b);
+    b->threads = kLanes * width;
     b->ctas = ctas;
     b->folds = batch_common_folds(b);
     {
@@ -1985,7 +2059,10 @@ int ngpu_batch_destroy(ngpu_batch* b) {
         batch_drop_graph(b);
         // members keep the batch's kernels until their next initialisation
         for (ngpu_sim* s : b->sims)
-            if (s->batch == b) s->batch = nullptr;
+            if (s->batch == b) {
+                s->batch = nullptr;
+                s->split_warps = 0;
+            }
     }
     delete b;
     return NGPU_OK;

@@ -1328,6 +1328,24 @@ __global__ void __launch_bounds__(kLanes * kMaxWarps, NGPU_ADV_MIN_BLOCKS)
     advance_body<R, MS, NoClasses>(B.sim[k], blockIdx.x - B.cta0[k], t0, n_steps, smem, ctr);
 }
 
+// A team's numbers into the layout of one CTA per group: its first copy of the
+// junction accumulators and segment links into jacc and sepv, the separators'
+// assembled rows to the other nodes' (A: the team's layout; a block per group).
+template <typename R>
+__global__ void k_leave_team(SimArgs<R> A, double* jacc, R* sepv) {
+    const int g = blockIdx.x, lane = threadIdx.x & 31;
+    const size_t nj = (size_t)2 * A.n_jslots * kLanes;
+    for (size_t t = threadIdx.x; t < nj; t += blockDim.x) jacc[g * nj + t] = A.jacc[3 * g * nj + t];
+    const Group<R> G = group_of(A, g);
+    const R* from = A.sepv + (size_t)g * 3 * kTeamRows * A.n_seps * kLanes + lane;
+    R* to = sepv + (size_t)g * 4 * A.n_seps * kLanes + lane;
+    for (int k = threadIdx.x >> 5; k < A.n_seps; k += blockDim.x >> 5) {
+        const R* f = from + (size_t)k * kTeamRows * kLanes;
+        for (int r = 0; r < 4; ++r) to[(size_t)(4 * k + r) * kLanes] = f[r * kLanes];
+        store_row(G, A.seps[k].node, f[4 * kLanes], f[5 * kLanes], f[6 * kLanes]);
+    }
+}
+
 // Parameter table: ptab[g][row][lane] = params[set][row_param[row]][row_sec[row]]
 // for instance g*32+lane = set*n_stim + stim (padding lanes repeat the last instance).
 __global__ void k_gather_params(const float* __restrict__ params, const int* __restrict__ row_param,
