@@ -1822,9 +1822,16 @@ static int sim_upload_nodes(ngpu_sim* s) {
         if (gs && !s->jit)
             return fail(NGPU_E_CUDA, "mechanism set '" + gs->name +
                                          "' runs only through runtime compilation: " + ngpu_jit::last_log());
-        if (!s->jit && s->layout == NGPU_LAYOUT_LANE_INSTANCE && s->n_warps > kMaxWarps)
-            return fail(NGPU_E_CUDA, "CTAs of more than " + std::to_string(kMaxWarps) +
-                                         " warps run only through runtime compilation: " + ngpu_jit::last_log());
+        if (!s->jit && s->layout == NGPU_LAYOUT_LANE_INSTANCE && s->n_warps > kMaxWarps) {
+            if (s->warps_chosen)
+                return fail(NGPU_E_CUDA, "CTAs of more than " + std::to_string(kMaxWarps) +
+                                             " warps run only through runtime compilation: " + ngpu_jit::last_log());
+            // the library's own choice gives way to what the ahead-of-time kernels run
+            const size_t plain = s->precision == NGPU_FP64 ? SmemPlan<double>::bytes(m->n) : SmemPlan<float>::bytes(m->n);
+            const int W = default_warps(m->n, kMaxWarps), ctas = std::min(3, ctas_by_smem(plain));
+            const int rc = s->initialized ? sim_narrow(s, W, ctas) : sim_split_again(s, W, ctas);
+            if (rc != NGPU_OK) return rc;
+        }
     }
     std::vector<int> uniq(s->n_rec_unique, -1);
     for (size_t r = 0; r < s->rec_nodes.size(); ++r) uniq[s->rec_cols[r]] = s->rec_nodes[r];
@@ -1966,9 +1973,14 @@ static int batch_select_kernels(ngpu_batch* b) {
     if (gs && !b->jit)
         return fail(NGPU_E_CUDA, "mechanism set '" + gs->name +
                                      "' runs only through runtime compilation: " + ngpu_jit::last_log());
-    if (!b->jit && b->threads > kLanes * kMaxWarps)
-        return fail(NGPU_E_CUDA, "CTAs of more than " + std::to_string(kMaxWarps) +
-                                     " warps run only through runtime compilation: " + ngpu_jit::last_log());
+    if (!b->jit && b->threads > kLanes * kMaxWarps) {
+        // the ahead-of-time kernels' CTAs; fewer warps share each member's items
+        b->threads = kLanes * kMaxWarps;
+        for (ngpu_sim* s : b->sims) {
+            s->n_warps = std::min(s->n_warps, kMaxWarps);
+            s->split_warps = std::min(s->split_warps, kMaxWarps);
+        }
+    }
     return NGPU_OK;
 }
 
