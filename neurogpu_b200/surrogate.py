@@ -87,11 +87,20 @@ class SurrogateMLP:
         return t.as_tensor(x, dtype=t.float32, device=self.dev).expand(*shape).contiguous()
 
     def _stats(self, mu, sd, n):
-        """(keeps, pointer, pointer) of standardisation vectors, or of none."""
+        """Standardisation of n columns as the kernels take it: two float32 vectors (or None, None for none).
+        Statistics of another type, or given per row, are None: they are applied in torch's arithmetic."""
         if mu is None:
-            return (), None, None
-        m, s = self._f32(mu, n), self._f32(sd, n)
-        return (m, s), _p(m), _p(s)
+            return None, None
+        t = self.torch
+        mu, sd = (t.as_tensor(x, device=self.dev) for x in (mu, sd))
+        if any(x.dtype != t.float32 or tuple(x.shape) not in ((), (1,), (n,), (1, 1), (1, n)) for x in (mu, sd)):
+            return None
+        return tuple(x.reshape(-1).expand(n).contiguous() for x in (mu, sd))
+
+    def _standardised(self, x, mu, sd, n):
+        """(x, mean, deviation): x itself with what the kernels are to apply to it, or x standardised and None, None."""
+        v = self._stats(mu, sd, n)
+        return ((x - mu) / sd, None, None) if v is None else (x, *v)
 
     def _workspace(self, M, train):
         n = int(_ffi.lib().ngpu_mlp_workspace_bytes(M, self.width, self.k_in, self.n_out_p, int(train)))
@@ -113,15 +122,16 @@ class SurrogateMLP:
         t = self.torch
         X = t.as_tensor(X, dtype=t.float32, device=self.dev)
         M = X.shape[0]
+        X, x_mu, x_sd = self._standardised(X, self.x_mu, self.x_sd, self.n_in)
         X = self._f32(X, M, self.n_in)
+        y_stats = self._stats(self.y_mu, self.y_sd, self.n_out)
+        y_mu, y_sd = y_stats or (None, None)
         out = t.empty(M, self.n_out, device=self.dev)
         ws, n = self._workspace(M, False)
-        kx, x_mu, x_sd = self._stats(self.x_mu, self.x_sd, self.n_in)
-        ky, y_mu, y_sd = self._stats(self.y_mu, self.y_sd, self.n_out)
         _ffi.check("ngpu_mlp_predict", _ffi.lib().ngpu_mlp_predict(
-            _p(X), M, self.n_in, x_mu, x_sd, _ptrs(self.Wb), _ptrs(self.b), self.width, self.k_in, self.n_out,
-            self.n_out_p, y_mu, y_sd, _p(ws), n, _p(out), self._stream()))
-        return out
+            _p(X), M, self.n_in, _p(x_mu), _p(x_sd), _ptrs(self.Wb), _ptrs(self.b), self.width, self.k_in, self.n_out,
+            self.n_out_p, _p(y_mu), _p(y_sd), _p(ws), n, _p(out), self._stream()))
+        return out if y_stats is not None else out * self.y_sd + self.y_mu
 
     def loss_and_grads(self, X, Y, weight=None):
         """Mean squared error on standardised targets and the gradients of
@@ -129,16 +139,17 @@ class SurrogateMLP:
         t = self.torch
         X = t.as_tensor(X, dtype=t.float32, device=self.dev)
         M = X.shape[0]
+        Y = t.as_tensor(Y, dtype=t.float32, device=self.dev)
+        X, x_mu, x_sd = self._standardised(X, self.x_mu, self.x_sd, self.n_in)
+        Y, y_mu, y_sd = self._standardised(Y, self.y_mu, self.y_sd, self.n_out)
         X, Y = self._f32(X, M, self.n_in), self._f32(Y, M, self.n_out)
         if weight is not None:
             weight = self._f32(weight, M)
         ws, n = self._workspace(M, True)
-        kx, x_mu, x_sd = self._stats(self.x_mu, self.x_sd, self.n_in)
-        ky, y_mu, y_sd = self._stats(self.y_mu, self.y_sd, self.n_out)
         loss = t.empty((), device=self.dev)
         gW, gb = [t.empty(w.shape, device=self.dev) for w in self.W], [t.empty(b.shape, device=self.dev) for b in self.b]
         _ffi.check("ngpu_mlp_grads", _ffi.lib().ngpu_mlp_grads(
-            _p(X), _p(Y), _p(weight), M, self.n_in, x_mu, x_sd, y_mu, y_sd, _ptrs(self.Wb), _ptrs(self.Wtb),
+            _p(X), _p(Y), _p(weight), M, self.n_in, _p(x_mu), _p(x_sd), _p(y_mu), _p(y_sd), _ptrs(self.Wb), _ptrs(self.Wtb),
             _ptrs(self.b), self.width, self.k_in, self.n_out, self.n_out_p, _p(ws), n, _p(loss), _ptrs(gW), _ptrs(gb),
             self._stream()))
         return loss, gW, gb
