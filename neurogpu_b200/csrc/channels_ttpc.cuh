@@ -58,7 +58,7 @@ template <typename R>
 NGPU_HD R efun(R z) {
     if constexpr (sizeof(R) == 4) {
         const R series = (R)1 - z * (R)0.5 + efun_even(z);
-        const R direct = Math<R>::dv(z, Math<R>::ex(z) - (R)1);
+        const R direct = Math<R>::dvn(z, Math<R>::ex1(z) - (R)1);  // used from |z| = 1/2 on
         return fabs(z) < (R)0.5 ? series : direct;
     } else {
         if (fabs(z) < (R)1e-2) return (R)1 - z * ((R)0.5 - z * (R)(1.0 / 12.0));
@@ -76,8 +76,8 @@ NGPU_HD void efun_pair(R z, R& pos, R& neg) {
     const R a = fabs(z);
     if constexpr (sizeof(R) == 4) {
         const R c = efun_even(z), h = z * (R)0.5;
-        const R e = Math<R>::ex(fmin(a, (R)80));
-        const R small = Math<R>::dv(a, e - (R)1), big = small * e;
+        const R e = Math<R>::ex1(fmin(a, (R)80));
+        const R small = Math<R>::dvn(a, e - (R)1), big = small * e;
         const bool near0 = a < (R)0.5, up = z > (R)0;
         pos = near0 ? (R)1 - h + c : (up ? small : big);
         neg = near0 ? (R)1 + h + c : (up ? big : small);
@@ -97,7 +97,7 @@ NGPU_HD void efun_pair(R z, R& pos, R& neg) {
 // 1/(1 + e^z)
 template <typename R>
 NGPU_HD R sigm(R z) {
-    return Math<R>::rc((R)1 + Math<R>::ex(z));
+    return Math<R>::dvn((R)1, (R)1 + Math<R>::ex1(z));
 }
 // Gate with alpha/beta rates: returns xinf, sets *rate = qt*(alpha+beta) = 1/tau.
 template <typename R>
@@ -130,9 +130,9 @@ struct TTPCRates {
     static NGPU_HD void ca_lva(R v, R& mi, R& mr, R& hi, R& hr) {
         v = v + (R)10;
         mi = sigm((v + (R)30) * (R)(-1.0 / 6.0));
-        mr = qt * M::rc((R)5 + (R)20 * sigm((v + (R)25) * (R)(1.0 / 5.0)));
+        mr = qt * M::dvn((R)1, (R)5 + (R)20 * sigm((v + (R)25) * (R)(1.0 / 5.0)));
         hi = sigm((v + (R)80) * (R)(1.0 / 6.4));
-        hr = qt * M::rc((R)20 + (R)50 * sigm((v + (R)40) * (R)(1.0 / 7.0)));
+        hr = qt * M::dvn((R)1, (R)20 + (R)50 * sigm((v + (R)40) * (R)(1.0 / 7.0)));
     }
     // AllModels.cu:89-97
     static NGPU_HD void ih(R v, R& mi, R& mr) {
@@ -153,20 +153,20 @@ struct TTPCRates {
         mi = sigm(-(v + (R)1) * (R)(1.0 / 12.0));
         R mt = (v < (R)-50) ? (R)1.25 + (R)175.03 * M::ex(v * (R)0.026)
                             : (R)1.25 + (R)13 * M::ex(v * (R)-0.026);
-        mr = qt * M::rc(mt);
+        mr = qt * M::dvn((R)1, mt);
         hi = sigm((v + (R)54) * (R)(1.0 / 11.0));
         R z = (v + (R)75) * (R)(1.0 / 48.0);
-        hr = qt * M::rc((R)360 + ((R)1010 + (R)24 * (v + (R)55)) * M::ex(-(z * z)));
+        hr = qt * M::dvn((R)1, (R)360 + ((R)1010 + (R)24 * (v + (R)55)) * M::ex1(-(z * z)));
     }
     // AllModels.cu:121-130
     static NGPU_HD void k_tst(R v, R& mi, R& mr, R& hi, R& hr) {
         v = v + (R)10;
         mi = sigm(-v * (R)(1.0 / 19.0));
         R zm = (v + (R)71) * (R)(1.0 / 59.0);
-        mr = qt * M::rc((R)0.34 + (R)0.92 * M::ex(-(zm * zm)));
+        mr = qt * M::dvn((R)1, (R)0.34 + (R)0.92 * M::ex1(-(zm * zm)));
         hi = sigm((v + (R)66) * (R)(1.0 / 10.0));
         R zh = (v + (R)73) * (R)(1.0 / 23.0);
-        hr = qt * M::rc((R)8 + (R)49 * M::ex(-(zh * zh)));
+        hr = qt * M::dvn((R)1, (R)8 + (R)49 * M::ex1(-(zh * zh)));
     }
     // AllModels.cu:131-151
     static NGPU_HD void nap(R v, R& mi, R& mr, R& hi, R& hr) {
@@ -201,12 +201,12 @@ struct TTPCRates {
     // AllModels.cu:188-193
     static NGPU_HD R sk_zinf(R ca) {
         if (ca < (R)1e-7) ca = ca + (R)1e-7;
-        return M::rc((R)1 + M::pw((R)0.00043 * M::rc(ca), (R)4.8));
+        return M::dvn((R)1, (R)1 + M::pw((R)0.00043 * M::rc(ca), (R)4.8));
     }
     // AllModels.cu:194-197
     static NGPU_HD void skv3(R v, R& mi, R& mr) {
         mi = sigm((v - (R)18.7) * (R)(-1.0 / 9.7));
-        mr = ((R)1 + M::ex((v + (R)46.56) * (R)(-1.0 / 44.14))) * (R)(1.0 / 4.0);
+        mr = ((R)1 + M::ex1((v + (R)46.56) * (R)(-1.0 / 44.14))) * (R)(1.0 / 4.0);
     }
 };
 

@@ -214,7 +214,7 @@ inline bool build_cubin(int ms, bool fp64, const std::vector<uint32_t>& masks, c
     }
     const std::string src = source(ms, fp64, masks, folds, complete, ti, adv_warps, adv_ctas, team);
     std::vector<std::string> opt_s = {"--gpu-architecture=sm_" + arch, "-std=c++17",
-                                      "-lineinfo", "--ftz=true"};  // see ngpu_math.cuh
+                                      "-lineinfo"};
     int vmaj = 0, vmin = 0;
     nv.version(&vmaj, &vmin);
     uint64_t h = 1469598103934665603ull;

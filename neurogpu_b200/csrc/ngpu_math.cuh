@@ -27,15 +27,32 @@ namespace ngpu {
 template <typename R> struct Math;
 
 // FP32 uses the SFU approximations on the device; a host build (tests only)
-// falls back to the C library.  The runtime-compiled kernels flush
-// subnormals (--ftz): without it each approximate exponential, logarithm,
-// division and reciprocal carries a range check and two rescalings, 12 % of
-// the TTPC-like kernel's time at 300 instances and 7 % at 12,288; outputs
-// were the same bits on every case compared (no rate, state or matrix entry
-// comes near 1e-38).
+// falls back to the C library.  Subnormal numbers count everywhere: parameters,
+// states and sums keep them.  An approximate exponential or quotient pays for
+// that with a range check and rescaling, so ex1 and dvn stand where neither
+// can matter, and give the same bits there (tests/test_subnormals.py compares
+// every float):
+//   ex1(x)    e^x for a sum with a term of 0.3 or more: a subnormal e^x or 0
+//             is the same sum
+//   dvn(a, b) a / b where a, b and the quotient are normal numbers, 0 or
+//             infinite, or the quotient is not used
+// ms with the general forms throughout / with these / with every subnormal
+// flushed: TTPC-like cell, 200 steps, 12,288 instances 88.1 / 80.5 / 77.7, 300
+// instances 6.63 / 6.42 / 6.42; HH cell, 12,288 instances, 200 steps 32.2 /
+// 31.1 / 29.0, 3,072 instances, 400 steps 21.1 / 20.3 / 20.1.
 template <> struct Math<float> {
 #ifdef __CUDA_ARCH__
     static NGPU_HD float ex(float x) { return __expf(x); }
+    static NGPU_HD float ex1(float x) {
+        float y;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.442695041f));  // 2^(x log2 e)
+        return y;
+    }
+    static NGPU_HD float dvn(float a, float b) {
+        float y;
+        asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+        return y;
+    }
     static NGPU_HD float lg(float x) { return __logf(x); }
     static NGPU_HD float dv(float a, float b) { return __fdividef(a, b); }
     static NGPU_HD float rc(float a) { return __fdividef(1.0f, a); }
@@ -43,10 +60,12 @@ template <> struct Math<float> {
     // exp(x) - 1: series below |x| = 1e-2 (truncation < x^5/120), where exp(x) - 1 cancels
     static NGPU_HD float em1(float x) {
         if (fabsf(x) < 1e-2f) return x * (1.0f + x * (0.5f + x * (0.16666667f + x * 0.041666668f)));
-        return __expf(x) - 1.0f;
+        return ex1(x) - 1.0f;
     }
 #else
     static NGPU_HD float ex(float x) { return expf(x); }
+    static NGPU_HD float ex1(float x) { return expf(x); }
+    static NGPU_HD float dvn(float a, float b) { return a / b; }
     static NGPU_HD float lg(float x) { return logf(x); }
     static NGPU_HD float dv(float a, float b) { return a / b; }
     static NGPU_HD float rc(float a) { return 1.0f / a; }
@@ -59,13 +78,15 @@ template <> struct Math<float> {
     // error < z^5/120 < 3e-10 relative.
     static NGPU_HD float one_minus_exp_neg(float z) {
         const float series = z * (1.0f - z * (0.5f - z * (0.16666667f - z * 0.041666668f)));
-        const float direct = 1.0f - ex(-z);
+        const float direct = 1.0f - ex1(-z);
         return z < 0.03125f ? series : direct;
     }
 };
 
 template <> struct Math<double> {
     static NGPU_HD double ex(double x) { return exp(x); }
+    static NGPU_HD double ex1(double x) { return exp(x); }
+    static NGPU_HD double dvn(double a, double b) { return a / b; }
     static NGPU_HD double lg(double x) { return log(x); }
     static NGPU_HD double dv(double a, double b) { return a / b; }
     static NGPU_HD double rc(double a) { return 1.0 / a; }

@@ -317,6 +317,10 @@ template <typename R>
 struct RowSum {
     R x, r;
 };
+// An item's contribution to a junction; nothing waits for the old value.
+__device__ __forceinline__ void add_junction(double* p, double x) {
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(p), "d"(x) : "memory");
+}
 template <typename R>
 __device__ __forceinline__ RowSum<R> junction_sum(double* ja, R x0, R cx, R r0, R cr) {
     RowSum<R> o;
@@ -324,6 +328,11 @@ __device__ __forceinline__ RowSum<R> junction_sum(double* ja, R x0, R cx, R r0, 
     o.r = (R)((double)r0 + (double)cr + ja[kLanes]);
     ja[0] = 0.0;
     ja[kLanes] = 0.0;
+    // keeps this a branch that most nodes jump over: predicated instead, its
+    // FP64 sums and conversions are issued at every node (HH cell, 12,288
+    // instances, 4 steps: 3.17 million FP64 instructions, 0.28 so; 3,072
+    // instances, 400 steps: 21.1 ms, 20.4 so)
+    __threadfence_block();
     return o;
 }
 
@@ -353,8 +362,8 @@ __device__ __forceinline__ void eliminate_node(const Group<R>& G, const NodeRec<
         carry_r = cr;
     } else {
         double* ja = G.jacc + (size_t)(2 * s.pslot) * kLanes;
-        atomicAdd(ja, (double)cx);
-        atomicAdd(ja + kLanes, (double)cr);
+        add_junction(ja, (double)cx);
+        add_junction(ja + kLanes, (double)cr);
         carry_x = 0;
         carry_r = 0;
     }
@@ -543,8 +552,8 @@ __device__ __forceinline__ void eliminate_spine_row(const Group<R>& G, const Nod
         k.w = -s.b * om;
     } else {
         double* ja = G.jacc + (size_t)(2 * s.pslot) * kLanes;  // the upper separator
-        atomicAdd(ja, (double)(-s.b * lam));
-        atomicAdd(ja + kLanes, (double)(e_i - s.b * rr));
+        add_junction(ja, (double)(-s.b * lam));
+        add_junction(ja + kLanes, (double)(e_i - s.b * rr));
         sv[kLanes] = s.b * om;  // B: row u's coupling to dV_l
         sv[0] = nl.a * k.P;              // A: row l's coupling to dV_u (alpha = P)
         sv[2 * kLanes] = -nl.a * k.del;  // added to l's excess
