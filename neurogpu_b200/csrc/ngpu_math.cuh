@@ -105,7 +105,6 @@ NGPU_HD R cnexp(R x, R xinf, R tau, R dt) {
 constexpr double kFaraday = 96485.309;
 constexpr double kDefCai = 5.e-5;
 constexpr double kDefCao = 2.;
-constexpr double kLogCao = 0.69314718055994530942;  // log(kDefCao)
 __host__ __device__ constexpr double ktf_of(double celsius) {
     return 1000. * 8.3134 * (celsius + 273.15) / kFaraday;
 }
