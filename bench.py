@@ -293,7 +293,7 @@ def run_uneven(args):
     for w in ws:
         m = Model(w.cell)
         res = autotune.tune_warps(m, w.params, w.amps, w.dts, w.stim_node, w.stim_area, w.rec_nodes, w.v_init,
-                                  candidates=(2, 4, 6, 8), steps=min(100, w.nt - 20), warmup=20)
+                                  steps=min(100, w.nt - 20), warmup=20)
         tuned[w.cell.n_nodes] = [res["n_warps"], res["items_per_warp"]]
         s = Simulator(m, w.n_sets, w.n_stim, "fp32", n_warps=res["n_warps"], items_per_warp=res["items_per_warp"])
         s.set_params(w.params)

@@ -34,9 +34,11 @@ _CACHE: dict[str, dict] = {}
 # candidate shapes: (warps per CTA, items per warp) of the lane layout and
 # (instances per CTA, items per instance) of the warp layout
 LANE_SHAPES = ((2, 2), (4, 2), (4, 3), (6, 3), (8, 2), (8, 3), (8, 4))
-# lane-layout CTAs of more than 8 warps, timed for batches of at most one
-# 32-instance group per SM (compiled then for one CTA per SM)
-WIDE_SHAPES = ((12, 2), (12, 3), (16, 2), (16, 3))
+# lane-layout CTAs of more than 8 warps: timed for batches of at most two
+# 32-instance groups per SM (compiled then for two CTAs per SM), and of at most
+# one (for one; a group may then take several CTAs)
+TWO_PER_SM_SHAPES = ((12, 1), (12, 2), (12, 3))
+WIDE_SHAPES = TWO_PER_SM_SHAPES + ((16, 1), (16, 2), (16, 3))
 SM_COUNT = 148
 WARP_SHAPES = ((1, 16), (1, 32), (1, 64), (2, 32), (4, 32), (8, 32))
 # the warp layout is timed up to this many instances (beyond, 32 instances
@@ -50,6 +52,16 @@ def _key(cell: CellModel, n_sets: int, n_stim: int, precision: str) -> str:
     for arr in (cell.parent, cell.a, cell.b, cell.cm, cell.mech_mask, cell.section):
         h.update(np.ascontiguousarray(arr).tobytes())
     return f"{h.hexdigest()[:16]}:{n_sets}:{n_stim}:{precision}"
+
+
+def _own_shape(model: Model, n_sets, n_stim, precision) -> tuple[int, int]:
+    """(warps per CTA, items per warp) of the library's own lane layout for this batch."""
+    sim = Simulator(model, n_sets, n_stim, precision)
+    try:
+        lay = sim.layout()
+        return lay["cta_warps"], lay["items"]
+    finally:
+        sim.close()
 
 
 def _time_shape(model: Model, n_sets, n_stim, precision, layout, W, k, params, amps, dts, stim_node, stim_area,
@@ -75,7 +87,8 @@ def _time_shape(model: Model, n_sets, n_stim, precision, layout, W, k, params, a
 def tune(model: Model | CellModel, params, amps, dts, stim_node: int, stim_area: float, rec_nodes,
          v_init: float, steps: int = 100, warmup: int = 20, precision: str = "fp32",
          lane_shapes=LANE_SHAPES, warp_shapes=WARP_SHAPES, cache_file: str | Path | None = None) -> dict:
-    """Times every candidate layout and shape on this batch and returns
+    """Times every candidate layout and shape on this batch (by default the
+    library's own choice among them) and returns
     {"layout": "lane" | "warp", "n_warps": W, "items_per_warp": k,
     "ms_per_step": {"lane:W:k" | "warp:W:k": ms}}, ready for
     Simulator(..., layout=, n_warps=, items_per_warp=).  params [n_sets, ...]
@@ -84,8 +97,11 @@ def tune(model: Model | CellModel, params, amps, dts, stim_node: int, stim_area:
     model = model if isinstance(model, Model) else Model(model)
     cell = model.cell
     n_sets, n_stim = int(np.asarray(params).shape[0]), int(np.asarray(amps).shape[0])
-    if lane_shapes is LANE_SHAPES and (n_sets * n_stim + 31) // 32 <= SM_COUNT:
-        lane_shapes = LANE_SHAPES + WIDE_SHAPES
+    if lane_shapes is LANE_SHAPES:
+        per_sm = -(-((n_sets * n_stim + 31) // 32) // SM_COUNT)
+        lane_shapes += {1: WIDE_SHAPES, 2: TWO_PER_SM_SHAPES}.get(per_sm, ())
+        own = _own_shape(model, n_sets, n_stim, precision)
+        lane_shapes += () if own in lane_shapes else (own,)
     lane_shapes = tuple((int(w), int(k)) for w, k in lane_shapes if 1 <= int(w) <= 16 and 1 <= int(k) <= 8)
     warp_shapes = tuple((int(w), int(k)) for w, k in warp_shapes if 1 <= int(w) <= 8 and 1 <= int(k) <= 512)
     if n_sets * n_stim > WARP_LAYOUT_MAX_INSTANCES:
@@ -112,16 +128,22 @@ def tune(model: Model | CellModel, params, amps, dts, stim_node: int, stim_area:
 
 
 def tune_warps(model: Model | CellModel, params, amps, dts, stim_node: int, stim_area: float, rec_nodes,
-               v_init: float, candidates=(2, 4, 6, 8), steps: int = 100, warmup: int = 20,
+               v_init: float, candidates=None, steps: int = 100, warmup: int = 20,
                precision: str = "fp32", cache_file: str | Path | None = None, items=(2, 3, 4)) -> dict:
-    """The lane layout's shape alone (up to 8 warps: the shapes a batch of
-    several morphologies runs): times each (warp count, items per warp) and
+    """The lane layout's shape alone (the shapes a batch of several
+    morphologies runs): times each (warp count, items per warp) and
     returns {"n_warps": W, "items_per_warp": k, "ms_per_step":
     {"W:k": ms}} (what a batch of several morphologies, which runs the lane
-    layout, needs per member)."""
-    shapes = [(int(W), int(k)) for W in sorted({int(w) for w in candidates if 1 <= int(w) <= 8})
+    layout, needs per member).  candidates: warp counts up to 8; by default 2,
+    4, 6 and 8, CTAs of 12 warps (which a batch of at most two groups per SM
+    runs), and the library's own choice up to those."""
+    shapes = [(int(W), int(k)) for W in sorted({int(w) for w in candidates or (2, 4, 6, 8) if 1 <= int(w) <= 8})
               for k in (sorted({int(i) for i in items if 1 <= int(i) <= 8}) if W > 1 else [1])]
-    cell = model.cell if isinstance(model, Model) else model
+    model = model if isinstance(model, Model) else Model(model)
+    cell = model.cell
+    if candidates is None:
+        own = _own_shape(model, int(np.asarray(params).shape[0]), int(np.asarray(amps).shape[0]), precision)
+        shapes += [x for x in dict.fromkeys(TWO_PER_SM_SHAPES + (own,)) if x not in shapes and x[0] <= 12]
     key = (_key(cell, int(np.asarray(params).shape[0]), int(np.asarray(amps).shape[0]), precision) + ":warps:" +
            ",".join(f"{w}.{k}" for w, k in shapes))
     _load(cache_file)

@@ -581,8 +581,12 @@ static int resident_ctas(size_t smem_plain, int n_groups) {
 }
 static int resident_warps(int ctas) { return ctas == 1 ? 16 : ctas == 2 ? 12 : 8; }
 
-// CTAs per SM that kernels for explicitly chosen wide CTAs are compiled for.
-static int wide_ctas_per_sm(int n_groups) { return n_groups <= kSmCount ? 1 : 3; }
+// CTAs per SM that kernels for explicitly chosen CTAs of more than 8 warps are
+// compiled for: as many as the library would lay out, where the warps fit.
+static int wide_ctas_per_sm(int warps, size_t smem_plain, int n_groups) {
+    const int ctas = resident_ctas(smem_plain, n_groups);
+    return warps <= resident_warps(ctas) ? ctas : 3;
+}
 
 __global__ void k_cluster_probe() {}  // never launched: its occupancy is asked for
 
@@ -1360,7 +1364,7 @@ int ngpu_sim_create_layout(ngpu_model* m, int32_t n_sets, int32_t n_stim, int32_
         W = n_warps;
         s->warps_chosen = true;
     }
-    if (s->warps_chosen) s->ctas = W > kMaxWarps ? wide_ctas_per_sm(s->n_groups) : std::min(3, ctas_by_smem(plain));
+    if (s->warps_chosen) s->ctas = W > kMaxWarps ? wide_ctas_per_sm(W, plain, s->n_groups) : std::min(3, ctas_by_smem(plain));
     W = std::min(W, m->n);
     s->n_warps = W;
     s->items_per_warp = default_items(W);
@@ -2024,7 +2028,8 @@ int ngpu_batch_create(ngpu_sim* const* sims, int32_t n, ngpu_batch** out) {
             width = std::max(width, s->n_warps);
             continue;
         }
-        const int W = default_warps(s->m->n, wide && !s->warps_chosen ? resident_warps(ctas) : kMaxWarps);
+        const int most = wide ? resident_warps(ctas) : kMaxWarps;
+        const int W = s->warps_chosen ? std::min(s->n_warps, most) : default_warps(s->m->n, most);
         width = std::max(width, W);
         if (W == s->n_warps && !s->team && s->ctas == ctas) continue;
         if (s->initialized) {
