@@ -497,6 +497,8 @@ struct ngpu_sim {
     int split_ctas = 0;           // ... and CTAs per SM (0 warps: stay)
     int* d_skel = nullptr;        // the staged skeleton's tables (part.skel)
     int* d_team_items = nullptr;
+    char* d_split = nullptr;      // the one allocation of d_jacc, d_jx, d_sepv and the split's tables
+    char* d_narrow = nullptr;     // ... of d_jacc and d_sepv after sim_narrow
     Partition part;
     double* d_jacc = nullptr;
     void* d_jx = nullptr;
@@ -1106,10 +1108,10 @@ int ngpu_model_split_info(const ngpu_model* m, int32_t n_warps, int32_t* perm, i
 
 static void sim_free(ngpu_sim* s) {
     if (!s) return;
-    void* ptrs[] = {s->d_nodes, s->d_vbuf, s->d_slab, s->d_ptab, s->d_scr, s->d_jacc, s->d_jx,
+    void* ptrs[] = {s->d_nodes, s->d_vbuf, s->d_slab, s->d_ptab, s->d_scr, s->d_split, s->d_narrow,
                     s->d_inst_stim, s->d_bad, s->d_row_param, s->d_row_sec, s->d_amps,
-                    s->d_dts, s->d_trace, s->d_tmp_out, s->d_comps, s->d_seps, s->d_sepv, s->d_prange,
-                    s->d_phash, s->d_params_in, s->d_skel, s->d_team_items};
+                    s->d_dts, s->d_trace, s->d_tmp_out, s->d_prange,
+                    s->d_phash, s->d_params_in};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (s->h_stage) cudaFreeHost(s->h_stage);
@@ -1197,38 +1199,41 @@ static void sim_split_lanes(ngpu_sim* s, bool teams = true) {
 // accumulators and dV slots, work items, separators and segment links,
 // (re)allocated for the split and its items and separators uploaded.
 static int sim_upload_split(ngpu_sim* s) {
-    void** old[] = {(void**)&s->d_jacc, (void**)&s->d_jx, (void**)&s->d_comps, (void**)&s->d_seps, &s->d_sepv,
-                    (void**)&s->d_skel, (void**)&s->d_team_items};
-    for (void** p : old)
-        if (*p) {
-            cudaFree(*p);
-            *p = nullptr;
-        }
+    for (char** p : {&s->d_split, &s->d_narrow}) {
+        cudaFree(*p);
+        *p = nullptr;
+    }
     const size_t G = (size_t)s->n_groups, L = kLanes, esz = s->precision == NGPU_FP64 ? 8 : 4;
     const size_t nj = std::max(1, s->part.n_jslots), ns = std::max<size_t>(1, s->part.seps.size());
-    int rc = NGPU_OK;
     const size_t copies = s->team ? 3 : 1, links = s->team ? kTeamRows : 4;  // see advance_body
-    if (!(s->d_jacc = (double*)dmalloc(copies * G * 2 * nj * L * sizeof(double), &rc))) return rc;
-    if (!(s->d_jx = dmalloc(G * nj * L * esz, &rc))) return rc;
-    if (!(s->d_comps = (DevComp*)dmalloc(sizeof(DevComp) * std::max<size_t>(1, s->part.comps.size()), &rc))) return rc;
-    if (!(s->d_seps = (DevSep*)dmalloc(sizeof(DevSep) * ns, &rc))) return rc;
-    if (!(s->d_sepv = dmalloc(copies * G * links * ns * L * esz, &rc))) return rc;
     std::vector<DevComp> dc;
     for (const Comp& c : s->part.comps) dc.push_back({c.r, c.u, c.l, c.lk, c.light_lo, c.light_hi});
     std::vector<DevSep> ds;
     for (size_t k = 0; k < s->part.seps.size(); ++k)
         ds.push_back({s->part.seps[k], s->part.sep_par[k], s->part.sep_comp[k], 0});
-    if (!dc.empty()) NGPU_CUDA(cudaMemcpy(s->d_comps, dc.data(), sizeof(DevComp) * dc.size(), cudaMemcpyHostToDevice));
-    NGPU_CUDA(cudaMemcpy(s->d_seps, ds.data(), sizeof(DevSep) * ds.size(), cudaMemcpyHostToDevice));
-    if (!s->part.skel.empty()) {
-        if (!(s->d_skel = (int*)dmalloc(sizeof(int) * s->part.skel.size(), &rc))) return rc;
-        NGPU_CUDA(cudaMemcpy(s->d_skel, s->part.skel.data(), sizeof(int) * s->part.skel.size(), cudaMemcpyHostToDevice));
-    }
-    if (s->team) {
-        const std::vector<int> ti = team_items(s->m, s->part, s->team);
-        if (!(s->d_team_items = (int*)dmalloc(sizeof(int) * ti.size(), &rc))) return rc;
-        NGPU_CUDA(cudaMemcpy(s->d_team_items, ti.data(), sizeof(int) * ti.size(), cudaMemcpyHostToDevice));
-    }
+    const std::vector<int> ti = s->team ? team_items(s->m, s->part, s->team) : std::vector<int>();
+    // one allocation and one copy: each more is a tenth of a small
+    // simulation's preparation
+    std::vector<char> tables;
+    auto add = [&](const auto& v) {
+        const size_t at = tables.size(), bytes = sizeof(v[0]) * v.size();
+        tables.resize(at + (bytes + 255) / 256 * 256);
+        if (bytes) std::memcpy(tables.data() + at, v.data(), bytes);
+        return at;
+    };
+    const size_t comps = add(dc), seps = add(ds), skel = add(s->part.skel), items = add(ti);
+    const size_t jacc = copies * G * 2 * nj * L * sizeof(double), jx = G * nj * L * esz;  // multiples of 128
+    const size_t sepv = copies * G * links * ns * L * esz;
+    int rc = NGPU_OK;
+    if (!(s->d_split = (char*)dmalloc(tables.size() + jacc + jx + sepv, &rc))) return rc;
+    NGPU_CUDA(cudaMemcpy(s->d_split, tables.data(), tables.size(), cudaMemcpyHostToDevice));
+    s->d_jacc = (double*)(s->d_split + tables.size());
+    s->d_jx = s->d_split + tables.size() + jacc;
+    s->d_sepv = s->d_split + tables.size() + jacc + jx;
+    s->d_comps = (DevComp*)(s->d_split + comps);
+    s->d_seps = (DevSep*)(s->d_split + seps);
+    s->d_skel = (int*)(s->d_split + skel);
+    s->d_team_items = s->team ? (int*)(s->d_split + items) : nullptr;
     return NGPU_OK;
 }
 
@@ -1256,30 +1261,24 @@ template <typename R>
 static int sim_narrow(ngpu_sim* s, int warps, int ctas) {
     if (s->team) {
         const size_t G = (size_t)s->n_groups, L = kLanes, nj = (size_t)s->part.n_jslots, ns = s->part.seps.size();
+        const size_t jacc = G * 2 * nj * L * sizeof(double);
         int rc = NGPU_OK;
-        double* jacc = (double*)dmalloc(G * 2 * nj * L * sizeof(double), &rc);
-        if (!jacc) return rc;
-        R* sepv = (R*)dmalloc(G * 4 * ns * L * sizeof(R), &rc);
-        cudaError_t e = cudaSuccess;
-        if (sepv) {
-            e = cudaDeviceSynchronize();  // (its steps may be on any stream)
-            if (e == cudaSuccess) {
-                k_leave_team<R><<<s->n_groups, 256>>>(make_args<R>(s), jacc, sepv);
-                g_launches++;
-                e = cudaGetLastError();
-            }
-            if (e == cudaSuccess) e = cudaDeviceSynchronize();
+        char* to = (char*)dmalloc(jacc + G * 4 * ns * L * sizeof(R), &rc);
+        if (!to) return rc;
+        cudaError_t e = cudaDeviceSynchronize();  // (its steps may be on any stream)
+        if (e == cudaSuccess) {
+            k_leave_team<R><<<s->n_groups, 256>>>(make_args<R>(s), (double*)to, (R*)(to + jacc));
+            g_launches++;
+            e = cudaGetLastError();
         }
-        if (!sepv || e != cudaSuccess) {
-            cudaFree(jacc);
-            cudaFree(sepv);
-            return sepv ? fail(NGPU_E_CUDA, std::string("split: ") + cudaGetErrorString(e)) : rc;
+        if (e == cudaSuccess) e = cudaDeviceSynchronize();
+        if (e != cudaSuccess) {
+            cudaFree(to);
+            return fail(NGPU_E_CUDA, std::string("split: ") + cudaGetErrorString(e));
         }
-        cudaFree(s->d_jacc);
-        cudaFree(s->d_sepv);
-        cudaFree(s->d_team_items);
-        s->d_jacc = jacc;
-        s->d_sepv = sepv;
+        s->d_narrow = to;
+        s->d_jacc = (double*)to;
+        s->d_sepv = to + jacc;
         s->d_team_items = nullptr;
         s->team = 0;
     }
