@@ -106,14 +106,25 @@ NGPU_HD void mainen_node(MK mk, R v, R dt, R* __restrict__ st, const float* __re
         kca_n = INIT ? mi : cnexp_rate(kca_n, mi, mr, dt);
         R gx = (R)1e-4 * tadj * g_kca * kca_n; Itot += gx * (v - (R)Mainen::kEk); Gtot += gx;
     }
-    // km AllModels.cu:140-146, kv :150-156 (same rate form).  An exponential for
-    // each rate of a pair: from one (efun_pair) the larger rate carries one more
-    // rounding, and V's error against FP64 grows by up to 45 % over the HH
-    // cells' runs of 40 to 400 steps (uneven batch, 100 steps: 1.76e-7 of V,
-    // 2.35e-7 from one) for 1 % of their time.
+    // km AllModels.cu:140-146, kv :150-156 (same rate form).  In FP32 an
+    // exponential for each rate of a pair: from one (efun_pair) the larger rate
+    // carries one more rounding, and V's error against FP64 grows by up to 45 %
+    // over the HH cells' runs of 40 to 400 steps (uneven batch, 100 steps:
+    // 1.76e-7 of V, 2.35e-7 from one) for 1 % of their time.  In FP64 two take 9 %
+    // longer, and the rounding is no one's concern.
+    auto rates = [](R z, R& pos, R& neg) {
+        if constexpr (sizeof(R) == 4) {
+            pos = efun(z);
+            neg = efun(-z);
+        } else {
+            efun_pair(z, pos, neg);
+        }
+    };
     auto kgate = [&](const R* p, R z, R& n) {
-        R a = p[3] * p[2] * efun(-z);
-        R b = p[4] * p[2] * efun(z);
+        R ep, en;
+        rates(z, ep, en);
+        R a = p[3] * p[2] * en;
+        R b = p[4] * p[2] * ep;
         mi = ab_gate(a, b, tadj, &mr);
         n = INIT ? mi : cnexp_rate(n, mi, mr, dt);
         R gx = (R)1e-4 * tadj * p[0] * n; Itot += gx * (v - (R)Mainen::kEk); Gtot += gx;
@@ -122,9 +133,10 @@ NGPU_HD void mainen_node(MK mk, R v, R dt, R* __restrict__ st, const float* __re
     if (mk & Mainen::kKv) kgate(kv, M::dv(v - kv[1], kv[2]), kv_n);
     if (mk & Mainen::kNa) {  // AllModels.cu:160-172, 266-273 (rates at v + vshift)
         R vm = v + (R)Mainen::kVshiftNa;
-        const R z = M::dv(vm - na[1], na[2]);
-        R a = na[3] * na[2] * efun(-z);
-        R b = na[4] * na[2] * efun(z);
+        R ep, en;
+        rates(M::dv(vm - na[1], na[2]), ep, en);
+        R a = na[3] * na[2] * en;
+        R b = na[4] * na[2] * ep;
         mi = ab_gate(a, b, tadj, &mr);
         a = na[11] * na[7] * efun(-M::dv(vm - na[5], na[7]));
         b = na[10] * na[7] * efun(M::dv(vm - na[6], na[7]));

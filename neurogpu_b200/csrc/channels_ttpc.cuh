@@ -69,8 +69,8 @@ NGPU_HD R efun(R z) {
 // the two is |z| / (e - 1) and the larger that times e.  Above 80, where e
 // may overflow FP32, the larger is |z| to well below FP64 rounding and the
 // smaller below 1e-30 (FP32 stops e's growth there).  The alpha/beta
-// pairs of NaTa_t, NaTs2_t and Nap_Et2's activation are efun of opposite
-// arguments.
+// pairs of NaTa_t, NaTs2_t, Nap_Et2's and (in FP64) the Mainen na, km, kv
+// activation are efun of opposite arguments.
 template <typename R>
 NGPU_HD void efun_pair(R z, R& pos, R& neg) {
     const R a = fabs(z);

@@ -830,6 +830,16 @@ __device__ __forceinline__ void load_separator(const Group<R>& G, const Skel<R>&
     K.sC[o] = vo[kLanes];
 }
 
+// Keeps the loads of all of these ahead of their first use.
+__device__ __forceinline__ void keep(float& a, float& b, float& c, float& d, float& e, float& f, float& g, double& h,
+                                     double& i) {
+    asm volatile("" : "+f"(a), "+f"(b), "+f"(c), "+f"(d), "+f"(e), "+f"(f), "+f"(g), "+d"(h), "+d"(i));
+}
+__device__ __forceinline__ void keep(double& a, double& b, double& c, double& d, double& e, double& f, double& g,
+                                     double& h, double& i) {
+    asm volatile("" : "+d"(a), "+d"(b), "+d"(c), "+d"(d), "+d"(e), "+d"(f), "+d"(g), "+d"(h), "+d"(i));
+}
+
 // S2 through shared memory.  Every warp stages a share of the separators
 // (their accumulated rows and couplings, and without a team in the first step
 // of a launch their voltages: one memory round trip for all of them).  The skeleton is
@@ -845,12 +855,8 @@ __device__ __forceinline__ void load_separator(const Group<R>& G, const Skel<R>&
 // the items themselves when a team of CTAs shares the tree.
 // team: the CTAs of a team each run the whole solve on the same numbers;
 // rd, clr: the junction accumulators this step reads and those it clears
-// (the same ones without a team).
-template <bool TEAM, typename T>
-__device__ __forceinline__ T ld_team(const T* p) {  // a team's numbers come from other SMs: read past the L1
-    if constexpr (TEAM) return __ldcg(p);
-    else return *p;
-}
+// (the same ones without a team; a team's come from other SMs and are read
+// past the L1).
 template <typename R, bool TEAM>
 __device__ __forceinline__ void skeleton_staged(const SimArgs<R>& A, const Group<R>& G, const NodeRec<R>* nr,
                                                 const Skel<R>& K, double* rd, double* clr, const R* sepv, bool load_v,
@@ -858,37 +864,81 @@ __device__ __forceinline__ void skeleton_staged(const SimArgs<R>& A, const Group
     using M = Math<R>;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int S = A.n_seps;
-#pragma unroll(TEAM ? 4 : 2)
-    for (int q = w; q < S; q += nw) {
-        const SkelNode sp = K.nd[q];
-        const NodeRec<R> s = nr[sp.node];
-        const size_t jo = (size_t)(2 * sp.jslot) * kLanes;
-        const R* sv = sepv + (size_t)sp.k * (TEAM ? kTeamRows : 4) * kLanes;
-        const R* row = TEAM ? sv + 4 * kLanes : G.scr + (size_t)sp.node * 3 * kLanes;
-        double x = (double)ld_team<TEAM>(row) + ld_team<TEAM>(rd + jo);
-        double rh = (double)ld_team<TEAM>(row + kLanes) + ld_team<TEAM>(rd + jo + kLanes);
-        R a = s.a, b = s.b, e = ld_team<TEAM>(row + 2 * kLanes);
-        const R la = ld_team<TEAM>(sv), lb = ld_team<TEAM>(sv + kLanes);
-        const R lx = ld_team<TEAM>(sv + 2 * kLanes), lr = ld_team<TEAM>(sv + 3 * kLanes);
-        if (sp.seg >= 0) {
-            a = la;
-            b = lb;
-            x += (double)lx;
-            rh += (double)lr;
-            e = 0;  // the segment already folded this node's axial term in
+    if constexpr (TEAM) {
+#pragma unroll 4
+        for (int q = w; q < S; q += nw) {
+            const SkelNode sp = K.nd[q];
+            const NodeRec<R> s = nr[sp.node];
+            const size_t jo = (size_t)(2 * sp.jslot) * kLanes;
+            const R* sv = sepv + (size_t)sp.k * kTeamRows * kLanes;
+            const R* row = sv + 4 * kLanes;
+            double x = (double)__ldcg(row) + __ldcg(rd + jo);
+            double rh = (double)__ldcg(row + kLanes) + __ldcg(rd + jo + kLanes);
+            R a = s.a, b = s.b, e = __ldcg(row + 2 * kLanes);
+            const R la = __ldcg(sv), lb = __ldcg(sv + kLanes);
+            const R lx = __ldcg(sv + 2 * kLanes), lr = __ldcg(sv + 3 * kLanes);
+            if (sp.seg >= 0) {
+                a = la;
+                b = lb;
+                x += (double)lx;
+                rh += (double)lr;
+                e = 0;  // the segment already folded this node's axial term in
+            }
+            if (rank == 0) {
+                clr[jo] = 0.0;
+                clr[jo + kLanes] = 0.0;
+            }
+            const int o = q * kLanes + lane;
+            K.acx[o] = x;
+            K.acr[o] = rh;
+            K.sA[o] = a;
+            K.sB[o] = b;
+            K.sE[o] = e;
         }
-        if (!TEAM || rank == 0) {
-            clr[jo] = 0.0;
-            clr[jo + kLanes] = 0.0;
+    } else {
+        // two separators' rows at a time, all loaded before any is used: left
+        // to itself the compiler waits for one row after the other (HH cell,
+        // 12,288 instances: 157 us per step, 142 so; TTPC-like 410 and 397)
+        constexpr int U = 2;
+        for (int q0 = w; q0 < S; q0 += U * nw) {
+            R rx[U], rr[U], e[U], la[U], lb[U], lx[U], lr[U];
+            double jx[U], jr[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int q = q0 + u * nw;
+                const SkelNode sp = K.nd[q < S ? q : q0];
+                const size_t jo = (size_t)(2 * sp.jslot) * kLanes;
+                const R* sv = sepv + (size_t)sp.k * 4 * kLanes;
+                const R* row = G.scr + (size_t)sp.node * 3 * kLanes;
+                rx[u] = row[0], rr[u] = row[kLanes], e[u] = row[2 * kLanes];
+                jx[u] = rd[jo], jr[u] = rd[jo + kLanes];
+                la[u] = sv[0], lb[u] = sv[kLanes];
+                lx[u] = sv[2 * kLanes], lr[u] = sv[3 * kLanes];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) keep(rx[u], rr[u], e[u], la[u], lb[u], lx[u], lr[u], jx[u], jr[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int q = q0 + u * nw;
+                if (q >= S) break;
+                const SkelNode sp = K.nd[q];
+                const NodeRec<R>& s = nr[sp.node];
+                const bool link = sp.seg >= 0;
+                double x = (double)rx[u] + jx[u], rh = (double)rr[u] + jr[u];
+                x += link ? (double)lx[u] : 0.0;
+                rh += link ? (double)lr[u] : 0.0;
+                const size_t jo = (size_t)(2 * sp.jslot) * kLanes;
+                clr[jo] = 0.0;
+                clr[jo + kLanes] = 0.0;
+                const int o = q * kLanes + lane;
+                K.acx[o] = x;
+                K.acr[o] = rh;
+                K.sA[o] = link ? la[u] : s.a;
+                K.sB[o] = link ? lb[u] : s.b;
+                K.sE[o] = link ? (R)0 : e[u];  // the segment already folded this node's axial term in
+                if (load_v) load_separator(G, K, q);
+            }
         }
-        const int o = q * kLanes + lane;
-        K.acx[o] = x;
-        K.acr[o] = rh;
-        K.sA[o] = a;
-        K.sB[o] = b;
-        K.sE[o] = e;
-        if constexpr (!TEAM)
-            if (load_v) load_separator(G, K, q);
     }
     __syncthreads();
     for (int l = A.n_lev - 1; l >= 0; --l) {
