@@ -184,8 +184,9 @@ int ngpu_sim_advance(ngpu_sim *s, int32_t t0, int32_t n_steps, void *cuda_stream
 int ngpu_sim_create_ex(ngpu_model *m, int32_t n_sets, int32_t n_stim, int32_t precision, int32_t n_warps,
                        ngpu_sim **out);
 /* As ngpu_sim_create_ex, also choosing how many work items per warp the tree
- * is split into (1..8; 0 = the library's choice: 3 for up to 8 warps, 1
- * above).  More items balance the warps'
+ * is split into (1..8; 0 = the library's choice: 3 for up to 8 warps, 2 for
+ * up to 12, 1 above, fewer where the skeleton's rows would not fit in shared
+ * memory beside them; ngpu_sim_layout tells the count in use).  More items balance the warps'
  * dynamic queue better at the price of more skeleton nodes; the best count
  * depends on the morphology, so the autotuner times it.  No counterpart in
  * the reference (one thread per compartment group, no split). */
@@ -195,11 +196,13 @@ int ngpu_sim_create_shaped(ngpu_model *m, int32_t n_sets, int32_t n_stim, int32_
  * As ngpu_sim_create with the layout chosen by the caller.
  *   NGPU_LAYOUT_LANE_INSTANCE  one lane per instance, 32 instances per CTA,
  *       cta_warps warps sharing the tree (1..16; above 8 only through the
- *       runtime-compiled kernel, bounded for 3 CTAs per SM), items work
- *       items per warp (1..8); 0 = the library's choice.  With up to 8 warps
- *       this is ngpu_sim_create_shaped.  Above 8 warps, a batch that leaves
- *       SMs idle shares each group's tree between a cluster of up to 8 such
- *       CTAs (one per SM).
+ *       runtime-compiled kernel, which is compiled for one CTA per SM of up
+ *       to 16 warps, two of up to 12 where the batch has that many, else for
+ *       three), items work items per warp (1..8); 0 = the library's choice,
+ *       which gives way to 8 warps where a runtime compilation fails.  With
+ *       up to 8 warps this is ngpu_sim_create_shaped.  Above 8 warps at one
+ *       CTA per SM, a batch that leaves SMs idle shares each group's tree
+ *       between a cluster of up to 8 such CTAs (one per SM).
  *       A B200 fills from about 148 x 32 x 2 instances on.
  *   NGPU_LAYOUT_WARP_INSTANCE  one warp per instance (its lanes share the
  *       instance's tree, split into `items` work items, 1..512; 0 = 32),
@@ -224,6 +227,9 @@ int ngpu_sim_layout(const ngpu_sim *s, int32_t *layout, int32_t *cta_warps, int3
  * same results).  Members keep their own parameters, stimuli, recordings and
  * traces (ngpu_sim_get_trace).  Up to 16 members.  The reference runs one
  * morphology per process (U/CudaStuff.cu:518-587); no counterpart.
+ * Members whose warps the library chose, or wider ones than the batch's CTAs,
+ * have their trees split for the batch; one that is already initialised keeps
+ * its split, and goes on from its state, until its next initialisation.
  *   ngpu_batch_init       ngpu_sim_init of every member, one launch
  *   ngpu_batch_advance    ngpu_sim_advance of every member, one launch
  *   ngpu_batch_run_graph  init + ceil(nt/chunk) advance launches captured once

@@ -42,13 +42,13 @@ struct FeatureArgs {
 
 // A trace is walked in stretches of time side by side: blocks of 32 traces
 // (lane = trace) and blockDim.y stretches.  Each stretch keeps what the whole
-// needs of it (FeatPart: extremes, sums, its first and last crossing, the
+// needs of it (the kF* rows in shared memory: extremes, sums, its first and last crossing, the
 // sums over the segments that start and end inside it, and the extremes of
 // the open pieces at its two ends); one warp joins the stretches in time
 // order, then every stretch counts its samples above half amplitude.
 //
 // What bounds it: reading the traces, and the window a second time.  10,000
-// traces of 3,168 samples (127 MB): 167 us with cold caches (103 us where a
+// traces of 3,168 samples (127 MB): 135 us, traces side by side (103 us where a
 // trace's samples lie side by side).  One thread per trace (the
 // form this replaces) took 0.49 ms: two warps per SM.
 constexpr int kFeatDoubles = 10, kFeatFloats = 9, kFeatInts = 3;

@@ -541,8 +541,10 @@ struct ngpu_sim {
 };
 
 // Work items per warp the tree is split into by default.  8-warp CTAs: 3
-// (ms per 200 steps at 12,288 instances with 1 / 2 / 3 / 4: TTPC-like 85.6 /
-// 83.6 / 77.6 / 83.3, HH 30.1 / 29.4 / 28.6 / 30.6).  12-warp CTAs: 2
+// (us per step at 12,288 instances with 1 / 2 / 3 / 4: TTPC-like 433 / 420 /
+// 388 / 423, HH cells of 500 compartments 148 / 138 / 133 / 134, of 800 245 /
+// 233 / 227 / 224; small trees in many groups take fewer: 128 compartments,
+// 51,200 instances 119 / 125 / 131 / 137).  12-warp CTAs: 2
 // (within 3 % of the best of 1 to 3 on four trees).  16-warp CTAs and teams:
 // 1, since a finer split lengthens the skeleton, which nothing hides there
 // (us per step with 1 / 2: HH cell, 33 instances 18.0 / 25.2; TTPC-like, 300
@@ -552,14 +554,17 @@ static int default_items(int n_warps) { return n_warps > 12 ? 1 : n_warps > 8 ? 
 // Thread-item layout: work items per instance at most / by default, and the
 // SM count the default CTA shape spreads a small batch over.
 constexpr int kMaxTiItems = 512;
-// Lane-instance CTAs of up to 16 warps (runtime-compiled kernels bounded for
-// 3 CTAs per SM; the ahead-of-time kernels take up to kMaxWarps).
+// Lane-instance CTAs of up to 16 warps (runtime-compiled kernels; the
+// ahead-of-time kernels take up to kMaxWarps).
 constexpr int kMaxWideWarps = 16;
 constexpr int kDefaultTiItems = 32;
 // Compartments per warp of a wide CTA: a passive cable of 50 takes 8.7 us per
 // step with 6 warps, 6.4 with 16; one of 128, 20 with 4 and 9.4 with 16.
 constexpr int kWideNodes = 3;
-// Compartments per warp of an 8-warp CTA.
+// Compartments per warp of an 8-warp CTA.  us per step with 16 / with 48:
+// HH cells of 50 compartments 25 / 39 (800 groups) and 79 / 77 (3,000), of 128
+// 71 / 88 and 252 / 233, of 300 177 / 205 and 645 / 669; passive cables of 50
+// 27 / 39 and 93 / 112, of 128 68 / 86 and 238 / 311, of 300 equal.
 constexpr int kNarrowNodes = 16;
 // Warps a tree gets by default out of the `most` its CTA could have.
 static int default_warps(int n_nodes, int most) {
@@ -574,10 +579,10 @@ static int ctas_by_smem(size_t smem) { return std::max(1, (int)((228 * 1024) / (
 // CTAs per SM a batch of lane-instance groups is laid out for: three of 8
 // warps, fewer and wider ones where the groups or their shared memory do not
 // fill three (24 warps at 80 registers either way; one CTA per SM takes 16
-// warps at 128 registers).  Measured on B200, 160 groups, us per step with
-// 8-warp CTAs and with 12-warp ones: HH cells of 200 / 800 / 1500 / 3000
-// compartments 63 / 169 / 316 / 653 and 43 / 143 / 261 / 537; the four
-// together as one batch (two CTAs by shared memory) 860 and 760.
+// warps at 128 registers).  Measured on B200, us per step with 8-warp CTAs (2
+// items per warp) and with 12-warp ones: HH cells of 200 / 800 / 1500 / 3000
+// compartments, 160 groups 38 / 152 / 291 / 615 and 35 / 131 / 244 / 507, 290
+// groups 44 / 181 / 360 / 761 and 38 / 162 / 324 / 718.
 static int resident_ctas(size_t smem_plain, int n_groups) {
     return std::min({3, ctas_by_smem(smem_plain), (n_groups + kSmCount - 1) / kSmCount});
 }

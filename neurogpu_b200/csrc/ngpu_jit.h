@@ -124,9 +124,8 @@ inline bool enabled() {
 // ti: also the thread-item layout's advance kernel.
 // team: the advance kernel is the one for clusters of CTAs (advance_body).
 // adv_warps: the advance kernels are bounded for CTAs of up to this many
-// warps; above 8, for adv_ctas CTAs per SM (3 CTAs: 10 warps 64 registers,
-// 12: 56, 16: 40; 1 CTA, for batches of at most one CTA per SM: 16 warps
-// 128 registers).
+// warps; above 8, for adv_ctas CTAs per SM (1 CTA: 16 warps 128 registers; 2:
+// 12 warps 80; 3: 10 warps 64, 12 warps 56, 16 warps 40).
 inline std::string source(int ms, bool fp64, const std::vector<uint32_t>& masks, const Folds& folds = {},
                           bool complete = false, bool ti = false, int adv_warps = 8, int adv_ctas = 3, bool team = false) {
     std::string list;

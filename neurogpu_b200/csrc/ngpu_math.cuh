@@ -37,9 +37,9 @@ template <typename R> struct Math;
 //   dvn(a, b) a / b where a, b and the quotient are normal numbers, 0 or
 //             infinite, or the quotient is not used
 // ms with the general forms throughout / with these / with every subnormal
-// flushed: TTPC-like cell, 200 steps, 12,288 instances 88.1 / 80.5 / 77.7, 300
-// instances 6.63 / 6.42 / 6.42; HH cell, 12,288 instances, 200 steps 32.2 /
-// 31.1 / 29.0, 3,072 instances, 400 steps 21.1 / 20.3 / 20.1.
+// flushed: TTPC-like cell, 200 steps, 12,288 instances 86.7 / 78.9 / 77.7, 300
+// instances 6.66 / 6.51 / 6.51; HH cell, 12,288 instances, 200 steps 30.5 /
+// 29.3 / 28.9, 3,072 instances, 400 steps 21.6 / 20.7 / 20.3.
 template <> struct Math<float> {
 #ifdef __CUDA_ARCH__
     static NGPU_HD float ex(float x) { return __expf(x); }

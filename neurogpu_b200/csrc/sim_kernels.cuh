@@ -688,7 +688,7 @@ __device__ __forceinline__ void backsub_store(const SimArgs<R>& A, const Group<R
 // HH cell 80.9 / 72.9, TTPC-like 259 / 228).  Not with
 // TI: thread-item layout (lanes on different items; no lane-0 prefetch), and
 // not in FP32 with
-// TEAM: teams run on at most half the SMs, their rows stay in L2, and the
+// TEAM: a team's batch is at most 74 groups, its rows stay in L2, and the
 // prefetch is instructions and a branch per block for nothing (without / with:
 // HH cell, 33 instances 17.5 / 18.0, 2,100 instances 29.0 / 30.1; TTPC-like,
 // 300 instances 32.6 / 34.0; in FP64 46.1 / 46.5 and 114 / 110, so FP64 keeps it).

@@ -124,8 +124,8 @@ def extract(v: torch.Tensor, dt: float, stim_on: float, stim_off: float) -> torc
 def extract_device(v: torch.Tensor, dt: float, stim_on: float, stim_off: float,
                    threshold: float = THRESHOLD) -> torch.Tensor:
     """extract() by the library's CUDA kernel (ngpu_trace_features): v [B, T]
-    float32 on the GPU, any strides; one thread per trace, both passes over
-    the trace in one launch."""
+    float32 on the GPU, any strides; both passes over the traces in one
+    launch."""
     import ctypes as C
 
     from . import _ffi

@@ -118,7 +118,7 @@ class Simulator:
                  n_warps: int = 0, items_per_warp: int = 0, layout: str = "lane"):
         """layout "lane" (one lane per instance, 32 instances per CTA; the
         default): n_warps warps per CTA share the tree (1..16; above 8 the
-        runtime-compiled kernel, bounded for 3 CTAs per SM), items_per_warp
+        runtime-compiled kernel), items_per_warp
         work items per warp (1..8).  layout "warp" (one warp per instance, for
         batches too small to fill the GPU): n_warps instances per CTA (1..8),
         items_per_warp the work items the instance's tree is split into

@@ -81,3 +81,29 @@ def test_late_ctas_change_nothing(ngpu_built, tmp_path, cell, precision):
         got[name] = _run(tmp_path, cell, precision, cache, name + "_out")
     np.testing.assert_array_equal(got["late"], got["level"])
     np.testing.assert_array_equal(got["level"][0], got["level"][2])
+
+
+# 60 steps from rest, before any spike: each step rounds V and a node's sums a few times (4e-6 mV each), in another
+# order for each split
+@pytest.mark.gpu
+@pytest.mark.parametrize("cell,n,sets", [("hh", 500, 11), ("hh", 161, 3), ("ttpc", 1501, 8), ("passive", 170, 70)])
+def test_teams_round_as_one_cta(ngpu_built, monkeypatch, cell, n, sets):
+    from neurogpu_b200 import configs
+    from neurogpu_b200.sim import Simulator
+    w = {"hh": lambda: configs.hh_active(n_sets=sets, t_stop=1.5, n_comp=n),
+         "ttpc": lambda: configs.ttpc_like(n_sets=sets, t_stop=1.5),
+         "passive": lambda: configs.passive_cable(n_sets=sets, t_stop=1.5, n_comp=n)}[cell]()
+    out = []
+    for team in (None, "0"):
+        if team is not None:
+            monkeypatch.setenv("NGPU_TEAM", team)
+        s = Simulator(w.cell, w.n_sets, w.n_stim, "fp32")
+        s.set_params(w.params)
+        s.set_stimulus(configs.step_amps([0.1 * (k + 1) for k in range(w.n_stim)], w.nt, w.dt, 0.25, 100.0), w.dts,
+                       w.stim_node, w.stim_area)
+        s.set_recording([0, n // 2, n - 1])
+        s.init(w.v_init)
+        s.advance(0, w.nt)
+        out.append(s.trace())
+        s.close()
+    np.testing.assert_allclose(out[0], out[1], rtol=0, atol=5e-4)
